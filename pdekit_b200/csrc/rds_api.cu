@@ -1121,8 +1121,8 @@ rds_status rds_finalize(rds_ctx *ctx)
       ctx->extra.push_back(g.d_tc);
       g.tune_tile[0] = 128; // one cell per TMEM lane
     }
-  // Euler 2D: lane-indexed tables of the cell kernels (FP64, and FP32 for the mixed form)
-  if (NEQ > 1 && d.dim == 2)
+  // Euler: lane-indexed tables of the cell kernels (FP64, and FP32 for the mixed form)
+  if (NEQ > 1)
     for (HostCellGroup &g : ctx->groups)
     {
       std::vector<double> lt;

@@ -1,0 +1,38 @@
+// Reciprocal and reciprocal square root in FP64 without branches, for chains that the compiler
+// should overlap between nodes or points: the library division and rsqrt branch on special
+// values, which keeps independent evaluations of an unrolled loop apart.
+//
+// Both start from the PTX approximations (relative error below 2^-19) and take one step of a
+// third-order iteration, so the error left is that of its own roundings (about one unit in the
+// last place; tests/cpp/math_test.cu). With e = 1 - x y the reciprocal is y / (1 - e), expanded
+// to y (1 + e + e^2); with e = 1 - x y^2 the reciprocal square root is y (1 - e)^(-1/2), expanded
+// to y (1 + e / 2 + 3 e^2 / 8) (Householder's iterations of order three).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace rds
+{
+
+// 1 / x for finite normal x; NaN where 1 / x is infinite, 0 or denormal.
+__device__ __forceinline__ double rcp_fast(double x)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
+
+// 1 / sqrt(x) for finite normal x > 0; NaN for other x.
+__device__ __forceinline__ double rsqrt_fast(double x)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(fma(e, 0.375, 0.5), y * e, y);
+}
+
+__device__ __forceinline__ float rcp_fast(float x) { return 1.f / x; }
+__device__ __forceinline__ float rsqrt_fast(float x) { return rsqrtf(x); }
+
+} // namespace rds
