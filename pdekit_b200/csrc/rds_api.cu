@@ -31,11 +31,15 @@ struct rds_ctx
   rds_desc desc{};
   int device             = 0;
   cudaStream_t stream    = nullptr;
-  cudaStream_t side      = nullptr; // boundary kernels, concurrent with the cell kernels
+  cudaStream_t side      = nullptr; // the first branch beside the main stream
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // one more side stream per further weak condition (they write disjoint slots, so they run
-  // concurrently with each other as well), with its join event
-  static constexpr int kMaxSides = 8;
+  // weak conditions launched together (indices into bcs), or each by itself where a strong one
+  // is among them
+  std::vector<std::vector<int>> bc_sets;
+  bool bc_strong = false;
+  // one more side stream per further set and per cell group after the first (they write disjoint
+  // slots, so they run concurrently), with its join event
+  static constexpr int kMaxSides = 12;
   cudaStream_t sides[kMaxSides] = {};
   cudaEvent_t ev_joins[kMaxSides] = {};
   bool own_stream        = false;
@@ -416,19 +420,30 @@ GatherArgs gather_args(rds_ctx *ctx, double cfl, const int *stop)
   return a;
 }
 
-// Side stream of the k-th weak condition (the first one is ctx->side).
+// Branches beside the main stream: the k-th set of weak conditions, then the cell groups after
+// the first (the first branch is ctx->side).
+int side_count(const rds_ctx *ctx)
+{
+  return std::min((int)ctx->bc_sets.size() + std::max(0, (int)ctx->groups.size() - 1),
+                  rds_ctx::kMaxSides);
+}
+
 cudaStream_t side_stream(rds_ctx *ctx, int k)
 {
-  const int n = std::min((int)ctx->bcs.size(), rds_ctx::kMaxSides);
-  k           = k % std::max(1, n);
+  k = k % std::max(1, side_count(ctx));
   return k == 0 ? ctx->side : ctx->sides[k];
 }
 
-// Forks the side streams of the conditions from the main stream (a parallel graph branch each
-// when captured).
+// Stream of cell group ig in a forked sweep: the main stream for the first.
+cudaStream_t group_stream(rds_ctx *ctx, int ig)
+{
+  return ig == 0 ? ctx->stream : side_stream(ctx, (int)ctx->bc_sets.size() + ig - 1);
+}
+
+// Forks the side streams from the main stream (a parallel graph branch each when captured).
 rds_status fork_sides(rds_ctx *ctx)
 {
-  const int n = std::min((int)ctx->bcs.size(), rds_ctx::kMaxSides);
+  const int n = side_count(ctx);
   RDS_CUDA(cudaEventRecord(ctx->ev_fork, ctx->stream));
   for (int k = 0; k < n; ++k)
     RDS_CUDA(cudaStreamWaitEvent(side_stream(ctx, k), ctx->ev_fork, 0));
@@ -438,7 +453,7 @@ rds_status fork_sides(rds_ctx *ctx)
 // Joins the side streams into the main stream.
 rds_status join_sides(rds_ctx *ctx)
 {
-  const int n = std::min((int)ctx->bcs.size(), rds_ctx::kMaxSides);
+  const int n = side_count(ctx);
   for (int k = 0; k < n; ++k)
   {
     cudaEvent_t e = k == 0 ? ctx->ev_join : ctx->ev_joins[k];
@@ -446,6 +461,33 @@ rds_status join_sides(rds_ctx *ctx)
     RDS_CUDA(cudaStreamWaitEvent(ctx->stream, e, 0));
   }
   return RDS_OK;
+}
+
+// Launches of one sweep's weak conditions and cells (the gather not counted).
+long long residual_launches(const rds_ctx *ctx)
+{
+  return (long long)ctx->groups.size() + (long long)ctx->bc_sets.size();
+}
+
+// Launches one set of conditions (indices into ctx->bcs) on stream s.
+rds_status launch_set(rds_ctx *ctx, const std::vector<int> &set, const int *stop, bool change,
+                      cudaStream_t s)
+{
+  const HostBC *bcs[kMaxBCSet];
+  BCArgs args[kMaxBCSet];
+  const int n = (int)set.size();
+  for (int k = 0; k < n; ++k)
+  {
+    bcs[k]  = &ctx->bcs[set[k]];
+    args[k] = bc_args(ctx, *bcs[k], stop);
+    if (change)
+      args[k].c32 = ctx->d_c32; // the change since the exact sweep, in FP32
+  }
+  return launch_on(ctx, s, [&](const char **name) {
+    return bcs[0]->desc.kind == RDS_BC_STRONG_DIRICHLET
+               ? launch_strong(args[0], ctx->desc.neq, s, name)
+               : launch_bc_set(bcs, args, n, ctx->desc.dim, ctx->desc.neq, s, name);
+  });
 }
 
 // Arguments of a correction sweep's cell kernel (defect-correction loop) for group ig.
@@ -477,37 +519,23 @@ rds_status launch_residual_kernels(rds_ctx *ctx, const int *stop)
 {
   const rds_desc &d = ctx->desc;
   // A strong Dirichlet condition writes the state that the cells read and that the conditions
-  // after it read: then the conditions run after the cells, in order, on the main stream.
-  bool strong = false;
-  for (const HostBC &b : ctx->bcs)
-    strong |= b.desc.kind == RDS_BC_STRONG_DIRICHLET;
+  // after it read: then the conditions run after the cells, in order, on the main stream (each
+  // set is then one condition).
   const bool with_bcs = !ctx->bcs.empty() && !ctx->no_bcs;
-  // per-kernel event timing: every kernel alone on the main stream, so that each event pair
+  // Per-kernel event timing: every kernel alone on the main stream, so that each event pair
   // brackets one kernel and not its overlap with the others (the results do not change: the
-  // conditions write their own slots)
-  const bool fork     = with_bcs && !strong && !ctx->timing;
-  // stream of the k-th condition: all on s (in order), or one side stream each when forked
-  auto launch_bcs = [&](cudaStream_t s, bool spread) -> rds_status {
-    for (size_t k = 0; k < ctx->bcs.size(); ++k)
-    {
-      const HostBC &b    = ctx->bcs[k];
-      const cudaStream_t sk = spread ? side_stream(ctx, (int)k) : s;
-      BCArgs a = bc_args(ctx, b, stop);
-      if (ctx->dc_phase == 2)
-        a.c32 = ctx->d_c32; // the change since the exact sweep, in FP32
-      rds_status st  = launch_on(ctx, sk, [&](const char **name) {
-        return launch_bc(b, a, b.physics, d.dim, d.neq, sk, name);
-      });
-      if (st != RDS_OK)
-        return st;
-    }
-    return RDS_OK;
-  };
+  // conditions and the groups write their own slots). Otherwise the conditions and the cell
+  // groups after the first run on branches of their own: small ones side by side, and of large
+  // ones the next group's blocks take the SMs that the last blocks of one leave (62,500 P3 cells,
+  // half triangles, half quadrilaterals: 373 -> 370 us a sweep; a batch's groups are small:
+  // enqueue_batch_iteration).
+  const bool side_bcs = with_bcs && !ctx->bc_strong && !ctx->timing;
+  const bool fork     = !ctx->timing && (side_bcs || ctx->groups.size() > 1);
   if (fork)
   {
     rds_status st = fork_sides(ctx);
-    if (st == RDS_OK)
-      st = launch_bcs(ctx->side, true);
+    for (size_t k = 0; st == RDS_OK && side_bcs && k < ctx->bc_sets.size(); ++k)
+      st = launch_set(ctx, ctx->bc_sets[k], stop, ctx->dc_phase == 2, side_stream(ctx, (int)k));
     if (st != RDS_OK)
       return st;
   }
@@ -515,20 +543,21 @@ rds_status launch_residual_kernels(rds_ctx *ctx, const int *stop)
   for (size_t ig = (size_t)ctx->grp_beg; ig < gend; ++ig)
   {
     const HostCellGroup &g = ctx->groups[ig];
+    const cudaStream_t sg  = fork ? group_stream(ctx, (int)ig) : ctx->stream;
     CellArgs a             = cell_args(ctx, g, stop);
     // programmatic dependent launch for the first cell group of a loop iteration (the kernel
     // before it on the stream is the previous iteration's gather)
     a.pdl = (ctx->loop_pdl && !ctx->timing && ig == 0) ? 1 : 0;
     if (ctx->dc_phase == 1 && g.scheme == RDS_PGB)
       a.theta = ctx->d_dc_theta + ctx->dc_cell_base[ig]; // blending coefficients at u_r
-    rds_status st          = launch(ctx, [&](const char **name) {
+    rds_status st          = launch_on(ctx, sg, [&](const char **name) {
       if (ctx->dc_phase == 2)
       {
         // correction sweep: the FP32 change of the cell residual since the exact sweep
         DcCellArgs da = dc_cell_args(ctx, ig, stop);
         da.pdl        = (ctx->loop_pdl && !ctx->timing && ig == 0) ? 1 : 0;
         bool ok       = false;
-        const cudaError_t e = launch_cells_scalar_dc(g, da, 0, 0, ctx->stream, name, &ok);
+        const cudaError_t e = launch_cells_scalar_dc(g, da, 0, 0, sg, name, &ok);
         return ok ? e : cudaErrorNotSupported;
       }
       if (ctx->active_precision == RDS_MIXED && ctx->use_tc && g.d_tc && !ctx->blend_on)
@@ -538,11 +567,10 @@ rds_status launch_residual_kernels(rds_ctx *ctx, const int *stop)
         const int grid   = std::max(1, std::min(ntiles, 4 * ctx->nsm));
         bool ok          = false;
         const cudaError_t e =
-            launch_cells_scalar_tc(g, a, false, grid, ntiles, ctx->stream, name, &ok);
+            launch_cells_scalar_tc(g, a, false, grid, ntiles, sg, name, &ok);
         return ok ? e : cudaErrorNotSupported;
       }
-      return launch_cells(g, a, g.physics, g.scheme, ctx->active_precision, d.dim, d.neq,
-                          ctx->stream, name);
+      return launch_cells(g, a, g.physics, g.scheme, ctx->active_precision, d.dim, d.neq, sg, name);
     });
     if (st != RDS_OK)
       return st;
@@ -550,17 +578,25 @@ rds_status launch_residual_kernels(rds_ctx *ctx, const int *stop)
     if (ctx->av_on && g.scheme == RDS_PGLDA)
     {
       const ViscArgs va = visc_args(ctx, ig, stop);
-      st                = launch(ctx, [&](const char **name) {
-        return launch_viscous(va, d.dim, d.neq, ctx->stream, name);
+      st                = launch_on(ctx, sg, [&](const char **name) {
+        return launch_viscous(va, d.dim, d.neq, sg, name);
       });
       if (st != RDS_OK)
         return st;
     }
   }
   if (fork)
-    return join_sides(ctx);
-  if (with_bcs)
-    return launch_bcs(ctx->stream, false);
+  {
+    const rds_status st = join_sides(ctx);
+    if (st != RDS_OK || side_bcs)
+      return st;
+  }
+  for (size_t k = 0; with_bcs && k < ctx->bc_sets.size(); ++k)
+  {
+    const rds_status st = launch_set(ctx, ctx->bc_sets[k], stop, ctx->dc_phase == 2, ctx->stream);
+    if (st != RDS_OK)
+      return st;
+  }
   return RDS_OK;
 }
 
@@ -1140,8 +1176,23 @@ rds_status rds_finalize(rds_ctx *ctx)
         ctx->extra.push_back(g.d_lt32);
       }
     }
-  // side streams of the weak conditions after the first (rds_ctx::sides)
-  for (int k = 1; k < std::min((int)ctx->bcs.size(), rds_ctx::kMaxSides); ++k)
+  // launches of the conditions: the weak ones of one physics and facet type together, in order;
+  // each by itself where a strong one is among them
+  for (const HostBC &b : ctx->bcs)
+    ctx->bc_strong |= b.desc.kind == RDS_BC_STRONG_DIRICHLET;
+  for (int k = 0; k < (int)ctx->bcs.size(); ++k)
+  {
+    size_t i = ctx->bc_strong ? ctx->bc_sets.size() : 0;
+    while (i < ctx->bc_sets.size() &&
+           (ctx->bc_sets[i].size() == kMaxBCSet ||
+            !same_bc_set(ctx->bcs[ctx->bc_sets[i][0]], ctx->bcs[k])))
+      ++i;
+    if (i == ctx->bc_sets.size())
+      ctx->bc_sets.emplace_back();
+    ctx->bc_sets[i].push_back(k);
+  }
+  // side streams after the first (rds_ctx::sides)
+  for (int k = 1; k < side_count(ctx); ++k)
   {
     RDS_CUDA(cudaStreamCreateWithFlags(&ctx->sides[k], cudaStreamNonBlocking));
     RDS_CUDA(cudaEventCreateWithFlags(&ctx->ev_joins[k], cudaEventDisableTiming));
@@ -2318,7 +2369,7 @@ static rds_status run_loop(rds_ctx *ctx, double cfl, int max_iter, double drop)
   if ((st = capture_chunk(ctx, gi, [&] { return enqueue_iteration(ctx, cfl, max_iter, drop); })) !=
       RDS_OK)
     return st;
-  const long long per_iter = (long long)ctx->groups.size() + (long long)ctx->bcs.size() + 1;
+  const long long per_iter = residual_launches(ctx) + 1;
   return replay_chunks(ctx, gi, (max_iter + chunk - 1) / chunk, per_iter * chunk);
 }
 
@@ -2453,7 +2504,7 @@ static rds_status run_loop_dc(rds_ctx *ctx, double cfl, int max_iter, double dro
   };
   if ((st = capture_graph(ctx, 6, cycles, cycle)) != RDS_OK)
     return st;
-  const long long per_sweep = (long long)ctx->groups.size() + (long long)ctx->bcs.size() + 1;
+  const long long per_sweep = residual_launches(ctx) + 1;
   const int per_graph       = cycles * m;
   const long long per_launch =
       fused ? (long long)cycles * (per_sweep + 1) : per_sweep * per_graph;
@@ -2583,7 +2634,7 @@ rds_status rds_run(rds_ctx *ctx, double cfl, int n)
   const int gi = ctx->active_precision == RDS_MIXED ? 4 : 3;
   if ((st = capture_graph(ctx, gi, 1, one)) != RDS_OK)
     return st;
-  const long long per_iter = (long long)ctx->groups.size() + (long long)ctx->bcs.size() + 1;
+  const long long per_iter = residual_launches(ctx) + 1;
   for (int i = 0; i < n; ++i)
   {
     RDS_CUDA(cudaGraphLaunch(ctx->graph_exec[gi], ctx->stream));
@@ -2646,7 +2697,7 @@ struct RkStage
 };
 
 static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc = 0,
-                                          const RkStage *rk = nullptr);
+                                          const RkStage *rk = nullptr, bool rebuild = true);
 
 // One RK3TVD step of every problem of a batched context (the stages of enqueue_rk3tvd over the
 // batch's persistent kernels, each problem with its own CFL).
@@ -2964,20 +3015,11 @@ rds_status rds_add_batch_bc(rds_ctx *ctx, const rds_bc_group *b, int physics)
   return st;
 }
 
-// One batched iteration: rebuild of the active lists (only after a phase change), boundary
-// facets of all problems on the side stream, persistent cell kernels over the active tiles of
-// each group (FP32 tiles and FP64 tiles in the mixed form), persistent gather with the
-// per-problem update, norm and stop test.
-// dc: 0 plain iteration (FP32 tiles of the problems in phase 0 when mixed, FP64 tiles of those
-// in phase 1); 1 exact sweep of the defect-correction loop (FP64 cells of every active problem,
-// blending coefficients kept for the corrections); 2 correction sweep (FP32 cell changes).
-static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc, const RkStage *rk)
+static RebuildArgs rebuild_args(rds_ctx *ctx)
 {
-  const rds_desc &d = ctx->desc;
-  const int P = ctx->nprob, G = (int)ctx->groups.size();
   RebuildArgs r{};
-  r.nprob       = P;
-  r.ngroups     = G;
+  r.nprob       = ctx->nprob;
+  r.ngroups     = (int)ctx->groups.size();
   r.phase       = ctx->d_phase;
   r.cbeg        = ctx->d_cbeg;
   r.cend        = ctx->d_cend;
@@ -2987,29 +3029,41 @@ static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc, cons
   r.nb_prefix   = ctx->d_nb_prefix;
   r.changed     = ctx->d_changed;
   r.stop        = ctx->d_stop;
-  rds_status st = launch(ctx, [&](const char **name) {
-    return launch_batch_rebuild(r, ctx->stream, name);
-  });
-  if (st != RDS_OK)
+  return r;
+}
+
+// One batched iteration: rebuild of the active lists (only after a phase change), boundary
+// facets of all problems on the side stream, persistent cell kernels over the active tiles of
+// each group (FP32 tiles and FP64 tiles in the mixed form), persistent gather with the
+// per-problem update, norm and stop test. The groups run side by side, each on a branch: with
+// them in line, a branch per condition and a rebuild every sweep, 128 sweeps of 24 problems of
+// 1,000-40,000 cells took 11.8 ms (9.1 now), 20 problems of 1,000-4,000 cells 847 ms to their
+// drops in the mixed form (590 now).
+// dc: 0 plain iteration (FP32 tiles of the problems in phase 0 when mixed, FP64 tiles of those
+// in phase 1); 1 exact sweep of the defect-correction loop (FP64 cells of every active problem,
+// blending coefficients kept for the corrections); 2 correction sweep (FP32 cell changes).
+static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc, const RkStage *rk,
+                                          bool rebuild)
+{
+  const rds_desc &d = ctx->desc;
+  const int P = ctx->nprob, G = (int)ctx->groups.size();
+  const RebuildArgs r = rebuild_args(ctx);
+  rds_status st = RDS_OK;
+  if (rebuild && (st = launch(ctx, [&](const char **name) {
+                    return launch_batch_rebuild(r, ctx->stream, name);
+                  })) != RDS_OK)
     return st;
-  const bool fork = !ctx->bcs.empty();
+  const bool fork = !ctx->timing && side_count(ctx) > 0;
   if (fork && (st = fork_sides(ctx)) != RDS_OK)
     return st;
-  for (size_t k = 0; k < ctx->bcs.size(); ++k)
-  {
-    const HostBC &b       = ctx->bcs[k];
-    const cudaStream_t sk = side_stream(ctx, (int)k);
-    BCArgs a              = bc_args(ctx, b, ctx->d_stop);
-    if (dc == 2)
-      a.c32 = ctx->d_c32; // the change since the exact sweep, in FP32
-    if ((st = launch_on(ctx, sk, [&](const char **name) {
-           return launch_bc(b, a, b.physics, d.dim, d.neq, sk, name);
-         })) != RDS_OK)
+  for (size_t k = 0; k < ctx->bc_sets.size(); ++k)
+    if ((st = launch_set(ctx, ctx->bc_sets[k], ctx->d_stop, dc == 2,
+                         fork ? side_stream(ctx, (int)k) : ctx->stream)) != RDS_OK)
       return st;
-  }
   for (int gi = 0; gi < G; ++gi)
   {
     const HostCellGroup &g = ctx->groups[gi];
+    const cudaStream_t sg  = fork ? group_stream(ctx, gi) : ctx->stream;
     if (dc == 2)
     {
       // correction sweep over the same active tiles as the exact sweep (phase 1)
@@ -3029,10 +3083,10 @@ static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc, cons
       da.stop       = ctx->d_stop;
       da.bt         = {ctx->d_tile_prefix + ((size_t)gi * 2 + 1) * (P + 1), g.d_cbeg, g.d_cend, P};
       const int grid = g.tune_grid[1] > 0 ? g.tune_grid[1] : 4 * ctx->nsm;
-      if ((st = launch(ctx, [&](const char **name) {
+      if ((st = launch_on(ctx, sg, [&](const char **name) {
              bool ok             = false;
              const cudaError_t e = launch_cells_scalar_dc(g, da, grid, g.tune_tile[1],
-                                                          ctx->stream, name, &ok);
+                                                          sg, name, &ok);
              return ok ? e : cudaErrorNotSupported;
            })) != RDS_OK)
         return st;
@@ -3046,12 +3100,12 @@ static rds_status enqueue_batch_iteration(rds_ctx *ctx, bool mixed, int dc, cons
         a.theta = ctx->d_dc_theta + ctx->dc_cell_base[gi];
       const int grid = g.tune_grid[ph] > 0 ? g.tune_grid[ph] : 4 * ctx->nsm;
       const bool tc  = ph == 0 && ctx->use_tc && g.d_tc;
-      if ((st = launch(ctx, [&](const char **name) {
+      if ((st = launch_on(ctx, sg, [&](const char **name) {
              bool ok = false;
              cudaError_t e =
-                 tc ? launch_cells_scalar_tc(g, a, true, grid, 0, ctx->stream, name, &ok)
+                 tc ? launch_cells_scalar_tc(g, a, true, grid, 0, sg, name, &ok)
                     : launch_cells_scalar_batch(g, a, ph == 0 ? RDS_MIXED : RDS_FP64, grid,
-                                                g.tune_tile[ph], ctx->stream, name, &ok);
+                                                g.tune_tile[ph], sg, name, &ok);
              return ok ? e : cudaErrorNotSupported;
            })) != RDS_OK)
         return st;
@@ -3134,11 +3188,12 @@ rds_status rds_iterate_batch(rds_ctx *ctx, int max_iter, double drop, int32_t *i
   const int total_iter = max_iter + 1;
   if (dc)
   {
-    const long long per_sweep = 2 + (long long)ctx->bcs.size() + (long long)ctx->groups.size();
+    const long long per_sweep = 1 + residual_launches(ctx);
     if (ctx->timing)
     {
       for (int it = 0; it < total_iter; ++it)
-        if ((st = enqueue_batch_iteration(ctx, mixed, it % m == 0 ? 1 : 2)) != RDS_OK)
+        if ((st = enqueue_batch_iteration(ctx, mixed, it % m == 0 ? 1 : 2, nullptr,
+                                          it == 0 || m == 1 || it % m == 1)) != RDS_OK)
           return st;
     }
     else
@@ -3147,7 +3202,10 @@ rds_status rds_iterate_batch(rds_ctx *ctx, int max_iter, double drop, int32_t *i
       auto cycle       = [&]() -> rds_status {
         for (int j = 0; j < m; ++j)
         {
-          const rds_status s2 = enqueue_batch_iteration(ctx, mixed, j == 0 ? 1 : 2);
+          // problems change phase in the exact sweep only: the active lists are rebuilt after it
+          // (and before the first sweep of the call, below)
+          const rds_status s2 = enqueue_batch_iteration(ctx, mixed, j == 0 ? 1 : 2, nullptr,
+                                                        m == 1 || j == 1);
           if (s2 != RDS_OK)
             return s2;
         }
@@ -3156,8 +3214,12 @@ rds_status rds_iterate_batch(rds_ctx *ctx, int max_iter, double drop, int32_t *i
       if ((st = capture_graph(ctx, 2, cycles, cycle)) != RDS_OK)
         return st;
       const int per_graph = cycles * m;
-      if ((st = replay_chunks(ctx, 2, (total_iter + per_graph - 1) / per_graph,
-                              per_sweep * per_graph)) != RDS_OK)
+      const RebuildArgs r = rebuild_args(ctx);
+      if ((st = launch(ctx, [&](const char **name) {
+             return launch_batch_rebuild(r, ctx->stream, name);
+           })) != RDS_OK ||
+          (st = replay_chunks(ctx, 2, (total_iter + per_graph - 1) / per_graph,
+                              per_sweep * per_graph + (m == 1 ? per_graph : cycles))) != RDS_OK)
         return st;
     }
   }
@@ -3173,7 +3235,7 @@ rds_status rds_iterate_batch(rds_ctx *ctx, int max_iter, double drop, int32_t *i
         RDS_OK)
       return st;
     const long long per_iter =
-        2 + (long long)ctx->bcs.size() + (long long)ctx->groups.size() * (mixed ? 2 : 1);
+        2 + residual_launches(ctx) + (mixed ? (long long)ctx->groups.size() : 0);
     if ((st = replay_chunks(ctx, 2, (total_iter + rds_ctx::kChunk - 1) / rds_ctx::kChunk,
                             per_iter * rds_ctx::kChunk)) != RDS_OK)
       return st;

@@ -299,8 +299,13 @@ struct GatherArgs
 // Cell residual kernels: dispatch over (physics, scheme, element type, order, precision).
 cudaError_t launch_cells(const HostCellGroup &g, const CellArgs &a, int physics, int scheme,
                          int precision, int dim, int neq, cudaStream_t s, const char **name);
-cudaError_t launch_bc(const HostBC &b, const BCArgs &a, int physics, int dim, int neq,
-                      cudaStream_t s, const char **name);
+// Weak conditions of one launch (same physics and facet type, same_bc_set); strong ones each have
+// their own.
+constexpr int kMaxBCSet = 8;
+bool same_bc_set(const HostBC &a, const HostBC &b);
+cudaError_t launch_bc_set(const HostBC *const *bcs, const BCArgs *args, int n, int dim, int neq,
+                          cudaStream_t s, const char **name);
+cudaError_t launch_strong(const BCArgs &a, int neq, cudaStream_t s, const char **name);
 // Node gather: mode bit 0 = compute dt, bit 1 = update u, bit 2 = norm partials, bit 3 = final
 // reduction; 16 / 17 = residual (17: and dt) followed by a Runge-Kutta stage combination.
 cudaError_t launch_gather(const GatherArgs &a, int mode, int nblocks, cudaStream_t s,
