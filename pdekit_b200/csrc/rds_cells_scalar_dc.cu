@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(NT)
       if (v == tid)
         dc_node_sweep(a.ga, v, ns);
       else
-        dc_correction_node<true>(a.ga, v);
+        dc_correction_node<true>(a.ga, v, a.ga.row[v], a.ga.row[v + 1]);
     }
     if (sweep + 1 < a.nsweeps && !sweep_barrier<CLUSTER>(a))
     {

@@ -24,26 +24,26 @@ __device__ __forceinline__ float dc_load_change(const float *p)
 }
 
 template <bool COHERENT>
-__device__ __forceinline__ void dc_correction_node(const GatherArgs &a, const int v)
+__device__ __forceinline__ void dc_correction_node(const GatherArgs &a, const int v, const int i0,
+                                                   const int i1)
 {
-  const int i0 = a.row[v], i1 = a.row[v + 1];
-  double sum   = 0.0;
-  int i        = i0;
-  constexpr int B = 4;
-  for (; i + B <= i1; i += B)
+  double *pu         = a.u + v;
+  const double u     = *pu, dres = a.dres[v];
+  const float dtv    = a.dtv[v];
+  double sum         = 0.0;
+  constexpr int B    = 4;
+  for (int i = i0; i < i1; i += B)
   {
     float c[B];
 #pragma unroll
-    for (int k = 0; k < B; ++k)
-      c[k] = dc_load_change<COHERENT>(a.c32 + __ldg(a.ent_slot + i + k));
+    for (int k = 0; k < B; ++k) // past the end: the first of the four again
+      c[k] = dc_load_change<COHERENT>(a.c32 + __ldg(a.ent_slot + (i + k < i1 ? i + k : i)));
 #pragma unroll
     for (int k = 0; k < B; ++k)
-      sum += double(c[k]);
+      if (i + k < i1)
+        sum += double(c[k]);
   }
-  for (; i < i1; ++i)
-    sum += double(dc_load_change<COHERENT>(a.c32 + __ldg(a.ent_slot + i)));
-  double *pu = a.u + v;
-  *pu        = *pu - (a.dres[v] + double(a.dtv[v]) * sum);
+  *pu = u - (dres + double(dtv) * sum);
 }
 
 // A node's correction-sweep data that stay the same within a cycle (its first kNodeCache entry
