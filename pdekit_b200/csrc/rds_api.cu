@@ -58,8 +58,11 @@ struct rds_ctx
   double *d_dt      = nullptr;
   double *d_vol     = nullptr;
   double *d_inv_vol = nullptr;
-  double *d_contrib = nullptr; // [neq][S]
-  double *d_wsc     = nullptr; // [W]
+  // contributions (struct Contrib): one equation, several equations
+  double *d_rec  = nullptr; // [E][2]
+  int32_t *d_pos = nullptr; // [S] entry of every slot (groups, then conditions)
+  double *d_val  = nullptr; // [neq][S]
+  double *d_wsc  = nullptr; // [W]
   double *d_stage   = nullptr; // AoS staging [nnodes*neq]
   int32_t *d_row = nullptr, *d_ent_slot = nullptr, *d_ent_ws = nullptr;
   double *d_part = nullptr, *d_norm = nullptr, *d_norm0 = nullptr, *d_hist = nullptr;
@@ -309,6 +312,25 @@ bool supported_physics(const rds_desc &d)
   }
 }
 
+// The contributions of a cell group or condition whose slots start at slot_base / ws_base.
+Contrib contrib(const rds_ctx *ctx, long long slot_base, long long ws_base)
+{
+  Contrib c{};
+  c.S         = ctx->S;
+  c.slot_base = slot_base;
+  if (ctx->desc.neq == 1)
+  {
+    c.rec = ctx->d_rec;
+    c.pos = ctx->d_pos + slot_base;
+  }
+  else
+  {
+    c.val = ctx->d_val;
+    c.wsc = ctx->d_wsc + ws_base;
+  }
+  return c;
+}
+
 CellArgs cell_args(rds_ctx *ctx, const HostCellGroup &g, const int *stop)
 {
   CellArgs a{};
@@ -319,11 +341,7 @@ CellArgs cell_args(rds_ctx *ctx, const HostCellGroup &g, const int *stop)
   a.X          = ctx->d_X;
   a.ngeo_nodes = ctx->desc.ngeo_nodes;
   a.u          = ctx->d_u;
-  a.contrib    = ctx->d_contrib;
-  a.S          = ctx->S;
-  a.slot_base  = g.slot_base;
-  a.wsc        = ctx->d_wsc;
-  a.ws_base    = g.ws_base;
+  a.out        = contrib(ctx, g.slot_base, g.ws_base);
   a.adv0       = ctx->desc.adv[0];
   a.adv1       = ctx->desc.adv[1];
   a.adv2       = ctx->desc.adv[2];
@@ -356,9 +374,7 @@ ViscArgs visc_args(rds_ctx *ctx, size_t ig, const int *stop)
   a.V          = t.vV;
   a.dV         = t.vdV;
   a.dVgeo      = t.vdVgeo;
-  a.contrib    = ctx->d_contrib;
-  a.S          = ctx->S;
-  a.slot_base  = g.slot_base;
+  a.out        = contrib(ctx, g.slot_base, g.ws_base);
   a.stop       = stop;
   return a;
 }
@@ -375,11 +391,7 @@ BCArgs bc_args(rds_ctx *ctx, const HostBC &b, const int *stop)
   a.nnodes     = ctx->desc.nnodes;
   a.gq         = b.d_gq;
   a.vol        = ctx->d_vol;
-  a.contrib    = ctx->d_contrib;
-  a.S          = ctx->S;
-  a.slot_base  = b.slot_base;
-  a.wsc        = ctx->d_wsc;
-  a.ws_base    = b.ws_base;
+  a.out        = contrib(ctx, b.slot_base, b.ws_base);
   a.adv0       = ctx->desc.adv[0];
   a.adv1       = ctx->desc.adv[1];
   a.gamma      = ctx->desc.gamma;
@@ -405,9 +417,7 @@ GatherArgs gather_args(rds_ctx *ctx, double cfl, const int *stop)
   a.row      = ctx->d_row;
   a.ent_slot = ctx->d_ent_slot;
   a.ent_ws   = ctx->d_ent_ws;
-  a.contrib  = ctx->d_contrib;
-  a.S        = ctx->S;
-  a.wsc      = ctx->d_wsc;
+  a.in       = contrib(ctx, 0, 0);
   a.vol      = ctx->d_vol;
   a.inv_vol  = ctx->d_inv_vol;
   a.res      = ctx->d_res;
@@ -1050,7 +1060,7 @@ rds_status rds_finalize(rds_ctx *ctx)
   const long long E = count[N];
   ctx->E            = E;
   std::vector<int32_t> pos(count.begin(), count.end() - 1);
-  std::vector<int32_t> ent_slot(E), ent_ws(E);
+  std::vector<int32_t> ent_slot(E), ent_ws(E); // slot and cell of an entry
   for (size_t ig = 0; ig < ctx->groups.size(); ++ig)
   {
     const HostCellGroup &g = ctx->groups[ig];
@@ -1090,7 +1100,9 @@ rds_status rds_finalize(rds_ctx *ctx)
   if ((st = dalloc(ctx, &ctx->d_u, (size_t)N * NEQ)) || (st = dalloc(ctx, &ctx->d_res, (size_t)N * NEQ)) ||
       (st = dalloc(ctx, &ctx->d_ws, N)) || (st = dalloc(ctx, &ctx->d_dt, N)) ||
       (st = dalloc(ctx, &ctx->d_vol, N)) || (st = dalloc(ctx, &ctx->d_inv_vol, N)) ||
-      (st = dalloc(ctx, &ctx->d_contrib, (size_t)S * NEQ)) || (st = dalloc(ctx, &ctx->d_wsc, W)) ||
+      (NEQ == 1 && ((st = dalloc(ctx, &ctx->d_rec, (size_t)E * 2)) || (st = dalloc(ctx, &ctx->d_pos, S)))) ||
+      (NEQ > 1 && (st = dalloc(ctx, &ctx->d_val, (size_t)S * NEQ))) ||
+      (st = dalloc(ctx, &ctx->d_wsc, W)) ||
       (st = dalloc(ctx, &ctx->d_stage, (size_t)N * NEQ)) || (st = dalloc(ctx, &ctx->d_row, N + 1)) ||
       (st = dalloc(ctx, &ctx->d_ent_slot, E)) || (st = dalloc(ctx, &ctx->d_ent_ws, E)) ||
       (st = dalloc(ctx, &ctx->d_part, (size_t)(ctx->gblocks + 1) * NEQ)) || // +1: two node ranges
@@ -1108,11 +1120,15 @@ rds_status rds_finalize(rds_ctx *ctx)
   RDS_CUDA(cudaMemsetAsync(ctx->d_stop, 0, sizeof(int), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
+  if (NEQ == 1)
+    RDS_CUDA(cudaMemsetAsync(ctx->d_rec, 0, (size_t)E * 2 * sizeof(double), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_wsc, 0, (size_t)W * sizeof(double), ctx->stream));
   if ((st = upload(ctx, ctx->d_row, count.data(), N + 1)) ||
       (st = upload(ctx, ctx->d_ent_slot, ent_slot.data(), E)) ||
       (st = upload(ctx, ctx->d_ent_ws, ent_ws.data(), E)))
     return st;
+  if (NEQ == 1) // where the cells and facets write their records
+    RDS_CUDA(launch_entry_of_slot((int)E, ctx->d_ent_slot, ctx->d_pos, ctx->stream));
 
   // Dual volumes: per-cell volume into the wave-speed slot space, then a gather (boundary
   // slots hold zero).
@@ -1139,6 +1155,11 @@ rds_status rds_finalize(rds_ctx *ctx)
   RDS_CUDA(launch_dual_volume(N, ctx->d_row, ctx->d_ent_ws, ctx->d_wsc, ctx->d_vol,
                               ctx->d_inv_vol, ctx->stream));
   RDS_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (NEQ == 1) // its wave speeds are in the records
+  {
+    cudaFree(ctx->d_wsc);
+    ctx->d_wsc = nullptr;
+  }
   if ((st = dalloc(ctx, &ctx->d_loop, 1)) != RDS_OK ||
       (st = dalloc(ctx, &ctx->d_stall, 1)) != RDS_OK)
     return st;
@@ -3445,7 +3466,8 @@ rds_status rds_destroy(rds_ctx *ctx)
   if (ctx->h_out)
     cudaStreamDestroy(ctx->h_out);
   void *bufs[] = {ctx->d_X,     ctx->d_u,     ctx->d_res,     ctx->d_ws,       ctx->d_dt,
-                  ctx->d_vol,   ctx->d_inv_vol, ctx->d_contrib, ctx->d_wsc,    ctx->d_stage,
+                  ctx->d_vol,   ctx->d_inv_vol, ctx->d_rec,     ctx->d_pos,    ctx->d_stage,
+                  ctx->d_val,   ctx->d_wsc,
                   ctx->d_row,   ctx->d_ent_slot, ctx->d_ent_ws, ctx->d_part,   ctx->d_norm,
                   ctx->d_norm0, ctx->d_hist,  ctx->d_iter,    ctx->d_stop,     ctx->d_zero,
                   ctx->d_status, ctx->d_counter, ctx->d_loop, ctx->d_rk_u1, ctx->d_rk_u2,

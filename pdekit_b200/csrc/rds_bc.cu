@@ -149,10 +149,10 @@ bc_points(const BCArgs &a, const FacetTables<double, D, NFDOF, NFQ, NFGEO> &tb, 
     const double scale = fabs(sum) > 1.e-14 ? total / sum : 1.0;
 #pragma unroll
     for (int n = 0; n < NFDOF; ++n)
-      a.contrib[e * a.S + a.slot_base + (long long)n * a.nfacets + f] = bres[n] * scale;
+      a.out.val[e * a.out.S + a.out.slot_base + (long long)n * a.nfacets + f] = bres[n] * scale;
   }
   for (int n = lane; n < NFDOF; n += G)
-    a.wsc[a.ws_base + (long long)n * a.nfacets + f] =
+    a.out.wsc[(size_t)n * a.nfacets + f] =
         a.vol[a.sol_conn[(size_t)n * a.nfacets + f]] * coeff;
 }
 

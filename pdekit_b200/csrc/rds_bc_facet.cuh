@@ -280,12 +280,13 @@ __device__ __forceinline__ void bc_weak_facet(const BCArgs &a,
   if (NEQ == 1 && a.c32)
   {
     // correction sweep of the defect-correction loop: the change since the exact sweep, whose
-    // contribution is still in contrib (FP64 difference, then FP32: relative to the change)
+    // contribution is still in the record (FP64 difference, then FP32: relative to the change)
 #pragma unroll
     for (int n = 0; n < NFDOF; ++n)
     {
-      const long long slot = a.slot_base + (long long)n * a.nfacets + f;
-      a.c32[slot]          = float(bres[n][0] - a.contrib[slot]);
+      const size_t i = (size_t)n * a.nfacets + f;
+      a.c32[a.out.slot_base + i] =
+          float(bres[n][0] - a.out.rec[(size_t)__ldg(a.out.pos + i) * 2]);
     }
   }
   else
@@ -293,11 +294,9 @@ __device__ __forceinline__ void bc_weak_facet(const BCArgs &a,
 #pragma unroll
     for (int n = 0; n < NFDOF; ++n)
     {
-      const long long slot = a.slot_base + (long long)n * a.nfacets + f;
-#pragma unroll
-      for (int e = 0; e < NEQ; ++e)
-        a.contrib[e * a.S + slot] = bres[n][e];
-      a.wsc[a.ws_base + (long long)n * a.nfacets + f] = a.vol[dof[n]] * coeff;
+      static_assert(NEQ == 1, "several equations: bc_points");
+      const int p = __ldg(a.out.pos + (size_t)n * a.nfacets + f);
+      reinterpret_cast<double2 *>(a.out.rec)[p] = make_double2(bres[n][0], a.vol[dof[n]] * coeff);
     }
   }
   if (bad)

@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(NT, 1) cells_euler(const __grid_constant__ Cel
       const int n = lane + s * G;
       if (n < NDOF)
       {
-        const long long slot0 = a.slot_base + (long long)n * a.ncells + c;
+        const long long slot0 = a.out.slot_base + (long long)n * a.ncells + c;
 #pragma unroll
         for (int e = 0; e < NEQ; ++e)
         {
@@ -930,13 +930,13 @@ __global__ void __launch_bounds__(NT, 1) cells_euler(const __grid_constant__ Cel
                                            : lda[s][e] + theta * diss[s][e];
           if (SCHEME == RDS_PGB && a.blend)
             r = skip ? lda[s][e] : lda[s][e] + tn[s] * diss[s][e];
-          a.contrib[e * a.S + slot0] = r; // write-back: the gather reads it from L2
+          a.out.val[e * a.out.S + slot0] = r; // write-back: the gather reads it from L2
         }
       }
     }
     if (lane == 0)
     {
-      a.wsc[a.ws_base + c] = vol * wmax;
+      a.out.wsc[c] = vol * wmax;
       if (SCHEME == RDS_PGB && a.theta)
         a.theta[c] = theta;
     }

@@ -14,7 +14,7 @@
 //                                               (src/solver/rdm/cellsplitters/PGLDA.hpp:171-310,
 //                                                PGN.hpp:154-289, PGB.hpp:314-498)
 //   wave speed |K| max_{q,n} max(1e-6, |k_n|)   (PGLDA.hpp:207-214,301-310)
-// and writes the cell's nodal residuals and wave speed to its contribution slots; the node
+// and writes the cell's nodal residuals and wave speed to its contribution records; the node
 // gather (rds_gather.cu) sums them in ascending cell order.
 //
 // Precision: T = double is the plain path. T = float evaluates interpolation, flux, upwind
@@ -220,7 +220,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
     }
   }
   // wave speed |K| max_{q,n} max(1e-6, |k_n|)
-  const T wsmax = fmax(T(1.e-6), kmax);
+  const double wsc = vol * double(fmax(T(1.e-6), kmax));
 
   double theta = 1.0;
   if (SCHEME == RDS_PGB)
@@ -234,7 +234,11 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
       a.theta[c] = theta;
   }
 
-  double *out = a.contrib + a.slot_base + c;
+  // the record of local node n: residual and wave speed, at its place in the node's list
+  auto put = [&](int n, double r) {
+    const int p = __ldg(a.out.pos + (size_t)n * a.ncells + c);
+    reinterpret_cast<double2 *>(a.out.rec)[p] = make_double2(r, wsc);
+  };
   if (EXT && SCHEME == RDS_PGB && a.blend)
   {
     // external nodal blending coefficient: theta_n of the cell's nodes, the N part dropped
@@ -249,7 +253,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
     const bool skip = tmax < 1.e-6;
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
-      out[(size_t)n * a.ncells] = skip ? lda[n] : lda[n] + tn[n] * diss[n];
+      put(n, skip ? lda[n] : lda[n] + tn[n] * diss[n]);
   }
   else if (SCHEME == RDS_PGPSI && fabs(phi) > 1.e-14)
   {
@@ -266,18 +270,14 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
     }
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
-      out[(size_t)n * a.ncells] = x[n] / sx * phi;
+      put(n, x[n] / sx * phi);
   }
   else
   {
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
-    {
-      const double r = (SCHEME == RDS_PGLDA) ? lda[n] : lda[n] + theta * diss[n];
-      out[(size_t)n * a.ncells] = r; // write-back: the gather reads it from L2
-    }
+      put(n, (SCHEME == RDS_PGLDA) ? lda[n] : lda[n] + theta * diss[n]);
   }
-  a.wsc[a.ws_base + c] = vol * double(wsmax);
 }
 
 // FP64 P3 Burgers cells: capped at 128 registers (4 blocks per SM instead of 3; 11 % faster,

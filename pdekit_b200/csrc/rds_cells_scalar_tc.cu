@@ -464,11 +464,11 @@ __global__ void __launch_bounds__(kTcCells)
     }
     if (live)
     {
-      double *out = a.contrib + a.slot_base + c;
+      const double wsc = vol * double(wsmax);
 #pragma unroll
       for (int n = 0; n < NDOF; ++n)
-        out[(size_t)n * a.ncells] = (SCHEME == RDS_PGLDA) ? lda[n] : lda[n] + theta * diss[n];
-      a.wsc[a.ws_base + c] = vol * double(wsmax);
+        reinterpret_cast<double2 *>(a.out.rec)[__ldg(a.out.pos + (size_t)n * a.ncells + c)] =
+            make_double2((SCHEME == RDS_PGLDA) ? lda[n] : lda[n] + theta * diss[n], wsc);
     }
     // TMEM is rewritten by the next tile's products: every lane's loads are complete here
     tc_fence_before();

@@ -104,15 +104,14 @@ __device__ __forceinline__ bool fp32_stalled(double rel, int it, StallRec *r, co
 // the FP32 change of its contribution since the exact sweep, u -= dt res + (dt / V) sum
 // (nothing else is written).
 //
-// The kernel waits on its chain of loads row -> entries -> contributions, so every load that does
-// not depend on the chain is issued before it (the stop flag too: its test waits with the row),
-// and a node's entries are taken B at a time, the last, partial B as well: their loads are all in
-// flight before the ordered sums consume them (an edge node of a P2 mesh has two entries; one
-// after the other they cost two chains). B by measurement, with the norm, update and stop test
-// (B200, one launch between events; one by one after groups of four before): 1,050,625 nodes of P2
-// triangles 34.0 us with 3, 33.3 with 2, 35.1 with 4 (36.0 before), P3 14.2 / 14.8 / 15.0 (14.7);
-// 423,000 Euler 2D nodes 25.0 with 2, 29.3 with 4 (31.2); 140,000 Euler 3D nodes, whose vertices
-// have 24 cells, 28.2 with 2, 25.8 with 4 (33.2).
+// The kernel waits on its chain of loads row -> (entries ->) contributions, so every load that
+// does not depend on the chain is issued before it (the stop flag too: its test waits with the
+// row), and a node's entries are taken B at a time, the last, partial B as well: their loads are
+// all in flight before the ordered sums consume them (an edge node of a P2 mesh has two entries;
+// one after the other they cost two chains). B by measurement, with the norm, update and stop test
+// (B200, one launch between events): 1,050,625 nodes of P2 triangles 25.3 us with 2, 27.2 with 3,
+// 28.8 with 4; 423,000 Euler 2D nodes 25.0 with 2, 29.3 with 4; 140,000 Euler 3D nodes, whose
+// vertices have 24 cells, 28.2 with 2, 25.8 with 4.
 template <int NEQ, bool DT, bool UPDATE, bool NORM, bool RK = false, int DC = 0>
 __device__ __forceinline__ void gather_node(const GatherArgs &a, const int v, const double cfl,
                                             double *sq)
@@ -120,171 +119,231 @@ __device__ __forceinline__ void gather_node(const GatherArgs &a, const int v, co
   static_assert(DC == 0 || NEQ == 1, "the defect-correction gather is scalar");
   const int stop = *a.stop;
   const int i0 = a.row[v], i1 = a.row[v + 1];
-  if (DC == 2)
+  if constexpr (DC == 2)
   {
     if (!stop)
       dc_correction_node<false>(a, v, i0, i1);
-    return;
   }
-  double acc[NEQ], un[NEQ];
-#pragma unroll
-  for (int e = 0; e < NEQ; ++e)
+  else
   {
-    acc[e] = 0.0;
-    un[e]  = UPDATE ? a.u[(size_t)e * a.nnodes + v] : 0.0;
-  }
-  double ws       = 0.0;
-  // 1 / V formed here (correctly rounded, the same value as the stored inverse) instead of
-  // loaded: one 8-byte read less per node; V itself is read once for both uses
-  const double vv = a.vol[v];
-  if (stop)
-    return;
-  const double iv = __drcp_rn(vv);
-  constexpr int B = NEQ == 1 ? 3 : NEQ == 4 ? 2 : 4;
-  for (int i = i0; i < i1; i += B)
-  {
-    int s[B], w[B];
+    double acc[NEQ], un[NEQ];
 #pragma unroll
-    for (int k = 0; k < B; ++k)
+    for (int e = 0; e < NEQ; ++e)
     {
-      const int j = i + k < i1 ? i + k : i; // past the end: the first of the four again
-      s[k]        = __ldg(a.ent_slot + j);
-      w[k]        = __ldg(a.ent_ws + j);
+      acc[e] = 0.0;
+      un[e]  = UPDATE ? a.u[(size_t)e * a.nnodes + v] : 0.0;
     }
-    double cv[B][NEQ], wv[B];
-#pragma unroll
-    for (int k = 0; k < B; ++k)
+    double ws       = 0.0;
+    // 1 / V formed here (correctly rounded, the same value as the stored inverse) instead of
+    // loaded: one 8-byte read less per node; V itself is read once for both uses
+    const double vv = a.vol[v];
+    if (stop)
+      return;
+    const double iv = __drcp_rn(vv);
+    constexpr int B  = NEQ == 5 ? 4 : 2;
+    for (int i = i0; i < i1; i += B)
     {
+      double cv[B][NEQ], wv[B];
+      if constexpr (NEQ == 1)
+      {
+#pragma unroll
+        for (int k = 0; k < B; ++k) // past the end: the first of the B again
+        {
+          const double2 t =
+              __ldcs(reinterpret_cast<const double2 *>(a.in.rec) + (i + k < i1 ? i + k : i));
+          cv[k][0] = t.x;
+          wv[k]    = t.y;
+        }
+      }
+      else
+      {
+        int s[B], w[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+        {
+          const int j = i + k < i1 ? i + k : i;
+          s[k]        = __ldg(a.ent_slot + j);
+          w[k]        = __ldg(a.ent_ws + j);
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+        {
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e)
+            cv[k][e] = __ldcs(a.in.val + e * a.in.S + s[k]);
+          wv[k] = __ldcs(a.in.wsc + w[k]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < B; ++k)
+        if (i + k < i1)
+        {
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e)
+            acc[e] = __dadd_rn(acc[e], __dmul_rn(iv, cv[k][e]));
+          ws = __dadd_rn(ws, wv[k]);
+        }
+    }
+    if (DC == 1)
+      a.ur[v] = un[0];
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e)
+      a.res[(size_t)e * a.nnodes + v] = acc[e];
+    a.ws[v] = ws;
+    if (RK)
+    {
+      // Runge-Kutta stage combination of solver/time/ExplicitTimeStepper.cpp:66-100, evaluated
+      // left to right without contraction like the reference's expression templates:
+      //   first stage   u_1 = u_n - dt * r
+      //   later stages  u_k = (ca * u_n + cb * u_s) - cc * (dt * r)
+      // dt is this stage's (first) or the first stage's (later stages; assemble_rhs keeps it)
+      const double d = DT ? __ddiv_rn(__dmul_rn(cfl, vv), ws) : a.dt[v];
+      if (DT)
+        a.dt[v] = d;
 #pragma unroll
       for (int e = 0; e < NEQ; ++e)
-        cv[k][e] = __ldcs(a.contrib + e * a.S + s[k]);
-      wv[k] = __ldcs(a.wsc + w[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < B; ++k)
-      if (i + k < i1)
       {
-#pragma unroll
-        for (int e = 0; e < NEQ; ++e)
-          acc[e] = __dadd_rn(acc[e], __dmul_rn(iv, cv[k][e]));
-        ws = __dadd_rn(ws, wv[k]);
+        const size_t k   = (size_t)e * a.nnodes + v;
+        const double r   = __dmul_rn(d, acc[e]);
+        const double un  = a.rk_un[k];
+        a.rk_out[k]      = a.rk_first ? __dsub_rn(un, r)
+                                      : __dsub_rn(__dadd_rn(__dmul_rn(a.rk_ca, un),
+                                                            __dmul_rn(a.rk_cb, a.rk_us[k])),
+                                                  __dmul_rn(a.rk_cc, r));
       }
-  }
-  if (DC == 1)
-    a.ur[v] = un[0];
-#pragma unroll
-  for (int e = 0; e < NEQ; ++e)
-    a.res[(size_t)e * a.nnodes + v] = acc[e];
-  a.ws[v] = ws;
-  if (RK)
-  {
-    // Runge-Kutta stage combination of solver/time/ExplicitTimeStepper.cpp:66-100, evaluated
-    // left to right without contraction like the reference's expression templates:
-    //   first stage   u_1 = u_n - dt * r
-    //   later stages  u_k = (ca * u_n + cb * u_s) - cc * (dt * r)
-    // dt is this stage's (first) or the first stage's (later stages; assemble_rhs keeps it)
-    const double d = DT ? __ddiv_rn(__dmul_rn(cfl, vv), ws) : a.dt[v];
+      return;
+    }
     if (DT)
-      a.dt[v] = d;
-#pragma unroll
-    for (int e = 0; e < NEQ; ++e)
     {
-      const size_t k   = (size_t)e * a.nnodes + v;
-      const double r   = __dmul_rn(d, acc[e]);
-      const double un  = a.rk_un[k];
-      a.rk_out[k]      = a.rk_first ? __dsub_rn(un, r)
-                                    : __dsub_rn(__dadd_rn(__dmul_rn(a.rk_ca, un),
-                                                          __dmul_rn(a.rk_cb, a.rk_us[k])),
-                                                __dmul_rn(a.rk_cc, r));
-    }
-    return;
-  }
-  if (DT)
-  {
-    const double dtv = __ddiv_rn(__dmul_rn(cfl, vv), ws);
-    a.dt[v]          = dtv;
-    if (DC == 1)
-    {
-      a.dres[v] = __dmul_rn(dtv, acc[0]); // this sweep's update, u_new = u - dres
-      a.dtv[v]  = float(dtv * iv);
-    }
-#pragma unroll
-    for (int e = 0; e < NEQ; ++e)
-    {
-      if (UPDATE)
-        a.u[(size_t)e * a.nnodes + v] = __dsub_rn(un[e], __dmul_rn(dtv, acc[e]));
-      if (NORM)
+      const double dtv = __ddiv_rn(__dmul_rn(cfl, vv), ws);
+      a.dt[v]          = dtv;
+      if (DC == 1)
       {
-        const double r = __dmul_rn(acc[e], dtv);
-        sq[e]          = __dmul_rn(r, r);
+        a.dres[v] = __dmul_rn(dtv, acc[0]); // this sweep's update, u_new = u - dres
+        a.dtv[v]  = float(dtv * iv);
+      }
+#pragma unroll
+      for (int e = 0; e < NEQ; ++e)
+      {
+        if (UPDATE)
+          a.u[(size_t)e * a.nnodes + v] = __dsub_rn(un[e], __dmul_rn(dtv, acc[e]));
+        if (NORM)
+        {
+          const double r = __dmul_rn(acc[e], dtv);
+          sq[e]          = __dmul_rn(r, r);
+        }
       }
     }
   }
 }
 
-template <int NEQ, bool DT, bool UPDATE, bool NORM, bool FINAL, bool RK = false, int DC = 0>
-__global__ void __launch_bounds__(kGBlock, NEQ == 1 ? 8 : 0) gather_nodes(const __grid_constant__ GatherArgs a)
+// Warp sums of NEQ values into smem [NEQ][kGBlock / 32] (the first half of block_sums; after a
+// barrier chunk_sum adds the warps' in order).
+template <int NEQ>
+__device__ __forceinline__ void warp_sums(const double (&v)[NEQ], double *smem)
 {
-  __shared__ double smem[NEQ * (kGBlock / 32)];
-  pdl_wait_and_release();
-  const int v = a.vbeg + blockIdx.x * blockDim.x + threadIdx.x;
-  double sq[NEQ];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int e = 0; e < NEQ; ++e)
-    sq[e] = 0.0;
-  const double cfl = DT && a.loop ? a.loop->cfl : a.cfl;
-  if (v < (a.vend > 0 ? a.vend : a.nnodes))
-    gather_node<NEQ, DT, UPDATE, NORM, RK, DC>(a, v, cfl, sq);
-  if (NORM)
   {
-    if (*a.stop) // uniform over the grid: only the last block of a launch sets it
-      return;
-    const double s = block_sums<kGBlock, NEQ>(sq, smem);
-    if (threadIdx.x < NEQ)
-      a.part[(size_t)(a.part_off + blockIdx.x) * NEQ + threadIdx.x] = s;
-    if (FINAL)
+    double t = v[e];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0)
+      smem[e * (kGBlock / 32) + warp] = t;
+  }
+}
+
+__device__ __forceinline__ double chunk_sum(const double *smem, int e)
+{
+  double s = 0.0;
+  for (int w = 0; w < kGBlock / 32; ++w)
+    s += smem[e * (kGBlock / 32) + w];
+  return s;
+}
+
+// Blocks of a gather launch that are resident on an SM (by their registers).
+constexpr int gather_blocks_per_sm(int neq) { return neq == 1 ? 8 : neq == 4 ? 4 : 3; }
+
+// A resident grid walks the chunks of kGBlock nodes (the norm's partial sums are per chunk). A
+// block per chunk instead waits out, chunk by chunk, two barriers and the fence and atomic of the
+// last-block test with its slots on the SM empty; here a chunk costs one barrier and a block one
+// fence (1,050,625 scalar nodes 33.2 -> 27.1 us a launch, 423,000 Euler 2D nodes 25.0 -> 21.1).
+template <int NEQ, bool DT, bool UPDATE, bool NORM, bool FINAL, bool RK = false, int DC = 0>
+__global__ void __launch_bounds__(kGBlock, gather_blocks_per_sm(NEQ))
+    gather_nodes(const __grid_constant__ GatherArgs a)
+{
+  __shared__ double smem[2][NEQ * (kGBlock / 32)];
+  pdl_wait_and_release();
+  const int vend   = a.vend > 0 ? a.vend : a.nnodes;
+  const int nchunk = (vend - a.vbeg + kGBlock - 1) / kGBlock;
+  const double cfl = DT && a.loop ? a.loop->cfl : a.cfl;
+  int buf          = 0;
+  for (int chunk = blockIdx.x; chunk < nchunk; chunk += gridDim.x, buf ^= 1)
+  {
+    const int v = a.vbeg + chunk * kGBlock + threadIdx.x;
+    double sq[NEQ];
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e)
+      sq[e] = 0.0;
+    if (v < vend)
+      gather_node<NEQ, DT, UPDATE, NORM, RK, DC>(a, v, cfl, sq);
+    if (NORM)
     {
-      // last-block-done: the block that finishes last reduces all partials (fixed order), so
-      // the norm needs no separate launch; no block ever waits for another
-      __shared__ bool last;
-      __shared__ double nv[kMaxNeq];
-      if (NEQ > 1)
-        __syncthreads(); // threads 0 .. NEQ - 1 have written the block's parts
-      if (threadIdx.x == 0)
+      if (*a.stop) // uniform over the grid: only the last block of a launch sets it
+        return;
+      warp_sums<NEQ>(sq, smem[buf]);
+      __syncthreads(); // the other buffer is free again: its sums were read before this barrier
+      if (threadIdx.x < NEQ)
+        a.part[(size_t)(a.part_off + chunk) * NEQ + threadIdx.x] =
+            chunk_sum(smem[buf], threadIdx.x);
+    }
+  }
+  if (NORM && FINAL)
+  {
+    // last-block-done: the block that finishes last reduces all partials (fixed order), so
+    // the norm needs no separate launch; no block ever waits for another
+    __shared__ bool last;
+    __shared__ double nv[kMaxNeq];
+    if (*a.stop)
+      return;
+    if (NEQ > 1)
+      __syncthreads(); // threads 0 .. NEQ - 1 have written the block's parts
+    if (threadIdx.x == 0)
+    {
+      __threadfence();
+      const unsigned done = atomicAdd(a.counter, 1u);
+      last                = (done == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (last)
+    {
+      __threadfence();
+      if (a.sq_out)
       {
-        __threadfence();
-        const unsigned done = atomicAdd(a.counter, 1u);
-        last                = (done == gridDim.x - 1);
-      }
-      __syncthreads();
-      if (last)
-      {
-        __threadfence();
-        if (a.sq_out)
-        {
-          // partitioned form: the plain sum of the block sums (fixed order) for the caller
-          double t[NEQ];
+        // partitioned form: the plain sum of the chunk sums (fixed order) for the caller
+        double t[NEQ];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e)
+          t[e] = 0.0;
+        for (int b = threadIdx.x; b < nchunk; b += blockDim.x)
 #pragma unroll
           for (int e = 0; e < NEQ; ++e)
-            t[e] = 0.0;
-          for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-#pragma unroll
-            for (int e = 0; e < NEQ; ++e)
-              t[e] += a.part[(size_t)(a.part_off + b) * NEQ + e];
-          const double r = block_sums<kGBlock, NEQ>(t, smem);
-          if (threadIdx.x < NEQ)
-            a.sq_out[threadIdx.x] = r;
-        }
-        else
-        {
-          const int max_iter = a.loop ? a.loop->max_iter : a.max_iter;
-          const double drop  = a.loop ? a.loop->drop : a.drop;
-          reduce_final<NEQ>(a.part, gridDim.x, a.nnodes, a.norm, a.norm0, a.hist, a.iter,
-                            max_iter, drop, a.stop_w, a.status, smem, nv, a.stall, a.loop);
-        }
-        if (threadIdx.x == 0)
-          *a.counter = 0u;
+            t[e] += __ldcg(a.part + (size_t)(a.part_off + b) * NEQ + e);
+        const double r = block_sums<kGBlock, NEQ>(t, smem[0]);
+        if (threadIdx.x < NEQ)
+          a.sq_out[threadIdx.x] = r;
       }
+      else
+      {
+        const int max_iter = a.loop ? a.loop->max_iter : a.max_iter;
+        const double drop  = a.loop ? a.loop->drop : a.drop;
+        reduce_final<NEQ>(a.part, nchunk, a.nnodes, a.norm, a.norm0, a.hist, a.iter, max_iter,
+                          drop, a.stop_w, a.status, smem[0], nv, a.stall, a.loop);
+      }
+      if (threadIdx.x == 0)
+        *a.counter = 0u;
     }
   }
 }
@@ -465,6 +524,14 @@ __global__ void cell_volume_kernel(int ncells, int dim, int nq, int ngeo,
     vol += w[q] * det;
   }
   cvol[c] = vol;
+}
+
+// The entry of every slot (set-up only).
+__global__ void entry_of_slot(int n, const int32_t *ent_slot, int32_t *pos)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n)
+    pos[ent_slot[i]] = i;
 }
 
 __global__ void dual_volume_kernel(int nnodes, const int32_t *row, const int32_t *ent_ws,
@@ -708,28 +775,53 @@ __global__ void __launch_bounds__(1024) batch_rebuild(const __grid_constant__ Re
   }
 }
 
+// Blocks of a launch over nblocks chunks: what the GPU holds at once, or a block per chunk where
+// that would be less than two chunks each (549 chunks of Euler 3D nodes on 444 resident blocks:
+// 29.7 us, 25.5 with a block each).
+cudaError_t gather_grid(int neq, int nblocks, int *grid)
+{
+  static int nsm = 0;
+  if (nsm == 0)
+  {
+    int dev = 0, n = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+      e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess)
+      return e;
+    nsm = n;
+  }
+  const int most = nsm * gather_blocks_per_sm(neq);
+  *grid          = nblocks < 2 * most ? nblocks : most;
+  return cudaSuccess;
+}
+
 template <int NEQ>
 cudaError_t launch_gather_neq(const GatherArgs &a, int mode, int nblocks, cudaStream_t s)
 {
+  int grid            = 0;
+  const cudaError_t e = gather_grid(NEQ, nblocks, &grid);
+  if (e != cudaSuccess)
+    return e;
   switch (mode)
   {
   case 0:
-    gather_nodes<NEQ, false, false, false, false><<<nblocks, kGBlock, 0, s>>>(a);
+    gather_nodes<NEQ, false, false, false, false><<<grid, kGBlock, 0, s>>>(a);
     break;
   case 1:
-    gather_nodes<NEQ, true, false, false, false><<<nblocks, kGBlock, 0, s>>>(a);
+    gather_nodes<NEQ, true, false, false, false><<<grid, kGBlock, 0, s>>>(a);
     break;
   case 7:
-    gather_nodes<NEQ, true, true, true, false><<<nblocks, kGBlock, 0, s>>>(a);
+    gather_nodes<NEQ, true, true, true, false><<<grid, kGBlock, 0, s>>>(a);
     break;
   case 15:
-    return launch_kernel(gather_nodes<NEQ, true, true, true, true>, dim3(nblocks), dim3(kGBlock),
-                         0, s, a.pdl != 0, a);
+    return launch_kernel(gather_nodes<NEQ, true, true, true, true>, dim3(grid), dim3(kGBlock), 0, s,
+                         a.pdl != 0, a);
   case 16:
-    gather_nodes<NEQ, false, false, false, false, true><<<nblocks, kGBlock, 0, s>>>(a);
+    gather_nodes<NEQ, false, false, false, false, true><<<grid, kGBlock, 0, s>>>(a);
     break;
   case 17:
-    gather_nodes<NEQ, true, false, false, false, true><<<nblocks, kGBlock, 0, s>>>(a);
+    gather_nodes<NEQ, true, false, false, false, true><<<grid, kGBlock, 0, s>>>(a);
     break;
   default:
     return cudaErrorInvalidValue;
@@ -741,11 +833,15 @@ cudaError_t launch_gather_neq(const GatherArgs &a, int mode, int nblocks, cudaSt
 // correction sweep
 cudaError_t launch_gather_dc(const GatherArgs &a, int mode, int nblocks, cudaStream_t s)
 {
+  int grid            = 0;
+  const cudaError_t e = gather_grid(1, nblocks, &grid);
+  if (e != cudaSuccess)
+    return e;
   if (mode == 18)
-    return launch_kernel(gather_nodes<1, true, true, true, true, false, 1>, dim3(nblocks),
+    return launch_kernel(gather_nodes<1, true, true, true, true, false, 1>, dim3(grid),
                          dim3(kGBlock), 0, s, a.pdl != 0, a);
   if (mode == 19)
-    return launch_kernel(gather_nodes<1, false, false, false, false, false, 2>, dim3(nblocks),
+    return launch_kernel(gather_nodes<1, false, false, false, false, false, 2>, dim3(grid),
                          dim3(kGBlock), 0, s, a.pdl != 0, a);
   return cudaErrorInvalidValue;
 }
@@ -846,6 +942,12 @@ cudaError_t launch_cell_volume_raw(int ncells, int dim, int nq, int ngeo, const 
 {
   cell_volume_kernel<<<(ncells + kBlock - 1) / kBlock, kBlock, 0, s>>>(
       ncells, dim, nq, ngeo, geo_conn, X, ngeo_nodes, w, dVgeo, cvol);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_entry_of_slot(int n, const int32_t *ent_slot, int32_t *pos, cudaStream_t s)
+{
+  entry_of_slot<<<(n + kGBlock - 1) / kGBlock, kGBlock, 0, s>>>(n, ent_slot, pos);
   return cudaGetLastError();
 }
 

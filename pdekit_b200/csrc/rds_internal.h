@@ -168,6 +168,27 @@ struct RebuildArgs
   int *stop;
 };
 
+// Contributions between the cells, the facets and the node gather.
+// One equation: a record {residual, wave speed} per entry of the nodes' lists (CSR over nodes, in
+// the reference's accumulation order), written by the cell or facet at the entry's place (pos) and
+// read by the node in one run. The FP64 cell kernels have stores to spare, and the gather saves a
+// step of its chain of loads and whole 32-byte sectors moved for 8 bytes (1,050,625 nodes of P2
+// triangles: 235 MB through L2 before, gather 29.6 -> 25.6 us, cells 49.6 -> 47.6).
+// Several equations: arrays over (equation, local node, cell), which the gather reads through the
+// entries' slots. Records of 48 bytes written at scattered places cost the Euler cells more than
+// they saved the gather (P3 hybrid mesh 366 -> 375 us a sweep), and so did FP32 changes at their
+// entries the correction sweeps of the mixed loop (c32; 320 x 320 P2 squares 326 -> 340 ms).
+struct Contrib
+{
+  double *__restrict__ rec;        // one equation: [entries][2]
+  const int32_t *__restrict__ pos; // entry of (local node, cell or facet), SoA [ndof][n]
+  double *__restrict__ val;        // several: [neq][S], this group's slots start at slot_base
+  long long S;                     // total slots
+  long long slot_base;             // also the group's slots in c32
+  double *__restrict__ wsc;        // wave speeds: cells' [ncells], facets' [nfdof][nfacets]
+};
+
+
 // Arguments common to every cell kernel.
 struct CellArgs
 {
@@ -178,11 +199,7 @@ struct CellArgs
   const double *__restrict__ X;         // geometry coords SoA [dim][ngeo_nodes]
   int ngeo_nodes;
   const double *__restrict__ u; // state SoA [neq][nnodes]
-  double *__restrict__ contrib; // [neq][S], this group's slots start at slot_base
-  long long S;                  // total contribution slots
-  long long slot_base;
-  double *__restrict__ wsc; // wave-speed contributions, this group at ws_base
-  long long ws_base;
+  Contrib out;
   double adv0, adv1, adv2, gamma;
   unsigned *status;
   const int *stop; // nonzero: skip the work (converged loop)
@@ -227,11 +244,7 @@ struct BCArgs
   int nnodes;
   const double *__restrict__ gq; // [neq][nfq][nfacets]
   const double *__restrict__ vol;
-  double *__restrict__ contrib;
-  long long S;
-  long long slot_base;
-  double *__restrict__ wsc;
-  long long ws_base;
+  Contrib out;
   double adv0, adv1, gamma;
   double relax;      // WeakWall: 1 for P1 facets, 1/(3p) otherwise
   double params[4];  // WeakSubInlet: T_tot, p_tot; WeakSubOutlet: p_out
@@ -239,8 +252,8 @@ struct BCArgs
   const int *stop;
   double *u_strong; // strong Dirichlet: the state it overwrites (the same buffer as u)
   // correction sweep of the defect-correction loop (one equation): when set, the facet writes
-  // the change of its contribution since the exact sweep (still in contrib) to c32[slot]
-  // instead of contrib, and no wave speed
+  // the change of its contribution since the exact sweep (still in its record) to c32[slot]
+  // instead of the record
   float *c32;
 };
 
@@ -254,9 +267,7 @@ struct GatherArgs
   const int32_t *__restrict__ row;     // [nnodes+1]
   const int32_t *__restrict__ ent_slot; // [E]
   const int32_t *__restrict__ ent_ws;   // [E]
-  const double *__restrict__ contrib;   // [neq][S]
-  long long S;
-  const double *__restrict__ wsc;
+  Contrib in; // slot_base, pos unused
   const double *__restrict__ vol;
   const double *__restrict__ inv_vol;
   double *__restrict__ res; // SoA [neq][nnodes]
@@ -328,6 +339,7 @@ void euler_lane_tables(const HostCellGroup &g, int dim, std::vector<double> &out
 cudaError_t launch_cells_euler(const HostCellGroup &g, const CellArgs &a, int physics,
                                int scheme, int precision, cudaStream_t s, const char **name,
                                bool *ok);
+cudaError_t launch_entry_of_slot(int n, const int32_t *ent_slot, int32_t *pos, cudaStream_t s);
 cudaError_t launch_dual_volume(int nnodes, const int32_t *row, const int32_t *ent_ws,
                                const double *cvol, double *vol, double *inv_vol, cudaStream_t s);
 // Batch mode: persistent cell kernel of a scalar group over its active tiles (block = tile).
@@ -421,8 +433,7 @@ struct ViscArgs
   const int32_t *sol_conn, *geo_conn;
   const double *X, *u, *eps;
   const double *w, *V, *dV, *dVgeo; // [nq], [nq][ndof], [D][nq][ndof], [D][nq][ngeo]
-  double *contrib;
-  long long S, slot_base;
+  Contrib out;
   const int *stop;
 };
 struct SensorArgs

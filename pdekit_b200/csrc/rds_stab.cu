@@ -7,7 +7,7 @@
 //              res_n += w_q detJ_q eps_q grad phi_n . grad u_e(q)  for every equation e
 //              (src/solver/rdm/cellsplitters/PGLDA.hpp:245-256, the viscosity interpolated as
 //              in assembly/PGRDMExplicitCellWorker.hpp:519-533). Runs after the cell kernel of
-//              the group and adds to its contribution slots; G lanes per cell, on the points
+//              the group and adds to its contributions; G lanes per cell, on the points
 //              to form the gradient terms, then on the nodes to contract them (shared memory).
 //   sensor     the Persson-Peraire smoothness sensor of the first state component
 //              (src/solver/art_visc/ArtificialViscosity.hpp:300-455,
@@ -236,10 +236,15 @@ __global__ void __launch_bounds__(kBlock) viscous_cells(const ViscArgs a)
           for (int k = 0; k < D; ++k)
             acc[e] += gr[k] * S[e * D + k];
       }
-      const long long slot = a.slot_base + (long long)n * a.ncells + c;
+      const size_t i = (size_t)n * a.ncells + c;
+      if constexpr (NEQ == 1)
+        a.out.rec[(size_t)__ldg(a.out.pos + i) * 2] += acc[0];
+      else
+      {
 #pragma unroll
-      for (int e = 0; e < NEQ; ++e)
-        a.contrib[e * a.S + slot] += acc[e];
+        for (int e = 0; e < NEQ; ++e)
+          a.out.val[e * a.out.S + a.out.slot_base + i] += acc[e];
+      }
     }
 }
 
