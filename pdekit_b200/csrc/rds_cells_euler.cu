@@ -136,16 +136,6 @@ __device__ __forceinline__ double rsqrt_pos(double x)
 }
 __device__ __forceinline__ float rsqrt_pos(float x) { return x > 0.f ? rsqrtf(x) : 0.f; }
 
-// max(0, x), and x < y of numbers that are not negative. FP64: integer tests, since a comparison
-// would take a slot of the FP64 pipe, which bounds these kernels.
-__device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
-__device__ __forceinline__ float pos_part(float x) { return x > 0.f ? x : 0.f; }
-__device__ __forceinline__ bool less_pos(double x, double y)
-{
-  return __double_as_longlong(x) < __double_as_longlong(y);
-}
-__device__ __forceinline__ bool less_pos(float x, float y) { return x < y; }
-
 // The three numbers of K+ in direction g and its unit normal; returns max_k |lambda_k|.
 template <typename T, int D>
 struct UpwindK

@@ -22,6 +22,7 @@
 // and the nodal residual in FP64.
 
 #include "rds_internal.h"
+#include "rds_math.cuh"
 #include "rds_tables.cuh"
 
 namespace rds
@@ -30,12 +31,42 @@ namespace rds
 namespace
 {
 
+// Whether the FP64 quadrature loop is unrolled: P1, and P2 but for PGB, whose three sums a node
+// would spill 368 bytes (125,000 P2 cells, PGN: 16.7 us rolled, 14.9 unrolled; PGB on 524,288: 45.4
+// and 52.6); the P3 body overflows the instruction cache.
+constexpr bool unroll_fp64(int ndof, int scheme)
+{
+  return ndof == 3 || (ndof == 6 && scheme != RDS_PGB);
+}
+
+// A cell's nodes: all its index loads, in flight together (and with the kernel's stop flag).
+template <int NDOF, int NGEO>
+struct CellNodes
+{
+  int v[NDOF], g[NGEO];
+};
+
+template <int NDOF, int NGEO>
+__device__ __forceinline__ void load_nodes(const CellArgs &a, const int c,
+                                           CellNodes<NDOF, NGEO> &nodes)
+{
+#pragma unroll
+  for (int n = 0; n < NDOF; ++n)
+    nodes.v[n] = __ldg(a.sol_conn + (size_t)n * a.ncells + c);
+#pragma unroll
+  for (int g = 0; g < NGEO; ++g)
+    nodes.g[g] = __ldg(a.geo_conn + (size_t)g * a.ncells + c);
+}
+
+// The sums of two products below name their fused operation: left to the compiler it may fuse
+// either product, and the single and the batched kernel, whose loops it unrolls alike but not
+// into the same code, must give the same bits.
 // EXT: the external nodal blending coefficient may be set (single contexts; batched contexts
 // never hold one, and the branch costs their kernels registers)
 template <int PHYS, int SCHEME, typename T, int NDOF, int NQ, int NFL, int NGEO, bool EXT = true>
 __device__ __forceinline__ void scalar_cell(const CellArgs &a,
                                             const Tables<T, 2, NDOF, NQ, NFL, NGEO> &tb,
-                                            const int c)
+                                            const int c, const CellNodes<NDOF, NGEO> &nodes)
 {
   // FP32 form: states and coordinates enter as deviations from the cell's first node, taken in
   // FP64 (u_n - u_0, X_g - X_0); interpolants and fluxes are written in those deviations
@@ -50,8 +81,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
 #pragma unroll
   for (int n = 0; n < NDOF; ++n)
   {
-    const int v = __ldg(a.sol_conn + (size_t)n * a.ncells + c);
-    ud[n]       = __ldg(a.u + v);
+    ud[n]       = __ldg(a.u + nodes.v[n]);
     un[n]       = DEV ? T(ud[n] - ud[0]) : T(ud[n]);
   }
   const T u0 = T(ud[0]);
@@ -64,7 +94,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
 #pragma unroll
     for (int g = 0; g < NGEO; ++g)
     {
-      const int v     = __ldg(a.geo_conn + (size_t)g * a.ncells + c);
+      const int v     = nodes.g[g];
       const double xg = __ldg(a.X + v), yg = __ldg(a.X + a.ngeo_nodes + v);
       if (g == 0)
       {
@@ -84,7 +114,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
       J10 = J10 + tb.dVgeo[1][0][g] * X0[g];
       J11 = J11 + tb.dVgeo[1][0][g] * X1[g];
     }
-    detj            = J00 * J11 - J01 * J10;
+    detj            = fma(J00, J11, -(J01 * J10));
     const T inv_det = T(1) / detj;
     ij00            = inv_det * J11;
     ij11            = inv_det * J00;
@@ -100,7 +130,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
   // i.e. the flux is contracted with invJ once per node instead of once per node and point.
   // The values r_q (and Phi = sum_q w_q detJ r_q) are formed first, so the contracted flux is
   // dead before the upwind loop; the rolled FP64 loop keeps them in shared memory.
-  constexpr int QUNROLL = sizeof(T) == 8 ? 1 : NQ;
+  constexpr int QUNROLL = sizeof(T) == 8 && !unroll_fp64(NDOF, SCHEME) ? 1 : NQ;
   constexpr bool RQ_SHARED = QUNROLL == 1;
   __shared__ T s_rq[RQ_SHARED ? NQ * kBlock : 1];
   T rq_reg[RQ_SHARED ? 1 : NQ];
@@ -125,17 +155,17 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
         F0 = T(a.adv0) * s;
         F1 = T(a.adv1) * s;
       }
-      G0[f] = ij00 * F0 + ij10 * F1;
-      G1[f] = ij01 * F0 + ij11 * F1;
+      G0[f] = fma(ij00, F0, ij10 * F1);
+      G1[f] = fma(ij01, F0, ij11 * F1);
     }
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
     {
-      T r = tb.dVf[0][q][0] * G0[0] + tb.dVf[1][q][0] * G1[0];
+      T r = fma(tb.dVf[0][q][0], G0[0], tb.dVf[1][q][0] * G1[0]);
 #pragma unroll
       for (int f = 1; f < NFL; ++f)
-        r = r + tb.dVf[0][q][f] * G0[f] + tb.dVf[1][q][f] * G1[f];
-      const double wj = double(tb.w[q] * detj);
+        r = fma(tb.dVf[1][q][f], G1[f], fma(tb.dVf[0][q][f], G0[f], r));
+      const double wj = double(mul_rn(tb.w[q], detj));
       vol += wj;
       phi += wj * double(r);
       if constexpr (RQ_SHARED)
@@ -145,21 +175,32 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
     }
   }
 
-  double lda[NDOF], diss[NDOF];
+  // LDA part sum_q e_q r_q K+_n with e = w detJ / sum K+ (w detJ beta_n is e K+_n), and N part
+  //   sum_q e_q K+_n sum_m K+_m (u_n - u_m) = d_n W_n - X_n,  d_n = u_n - u_0,
+  //   W_n = sum_q w_q detJ K+_n,  X_n = sum_q e_q (sum_m K+_m d_m) K+_n,
+  // one operation per point, node and sum instead of the three of u_n sum K+ - sum K+_m u_m scaled
+  // and added; PGN and PGPSI, which only use the sum of the two parts, take it in one (acc1).
+  // B200, before and after this and the clip and reciprocal that keep off the FP64 pipe and its
+  // branches (rds_math.cuh): 524,288 P2 cells, PGB, 47.6 -> 43.7 us a launch; 65,522 P3 cells,
+  // PGN, 27.5 -> 24.9. The FP64 pipe is 60 % busy on the former, the rest mostly the wait for the
+  // state (indices, then values) at five blocks an SM; walking several cells a thread with the
+  // next one's indices read ahead spilled and took 52 us.
+  constexpr bool SPLIT = SCHEME == RDS_PGLDA || SCHEME == RDS_PGB; // the LDA part by itself
+  double acc1[NDOF], accx[NDOF], accw[NDOF], d[NDOF];
 #pragma unroll
   for (int n = 0; n < NDOF; ++n)
   {
-    lda[n]  = 0.0;
-    diss[n] = 0.0;
+    acc1[n] = accx[n] = accw[n] = 0.0;
+    d[n]    = ud[n] - ud[0];
   }
   T kmax = T(0);
 
-  // FP64: the quadrature loop stays rolled (the unrolled P3 body overflows the instruction
-  // cache); table entries are then indexed constant-bank loads. FP32: unrolled.
+  // FP64: the quadrature loop stays rolled for P3 and for P2 with both parts (unroll_fp64); table
+  // entries are then indexed constant-bank loads. FP32: unrolled.
 #pragma unroll QUNROLL
   for (int q = 0; q < NQ; ++q)
   {
-    const double wj = double(tb.w[q] * detj);
+    const double wj = double(mul_rn(tb.w[q], detj));
     double rq;
     if constexpr (RQ_SHARED)
       rq = double(s_rq[q * kBlock + threadIdx.x]);
@@ -186,41 +227,54 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
     }
 
     // upwind coefficients k_n = a . invJ^T grad_xi phi_n = dV[0][q][n] A + dV[1][q][n] B
-    const T A = ax * ij00 + ay * ij10;
-    const T B = ax * ij01 + ay * ij11;
+    const T A = fma(ax, ij00, ay * ij10);
+    const T B = fma(ax, ij01, ay * ij11);
     T kp[NDOF];
     T sumkp = T(0);
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
     {
-      const T k = tb.dV[0][q][n] * A + tb.dV[1][q][n] * B;
-      kp[n]     = k > T(0) ? k : T(0);
+      const T k = fma(tb.dV[0][q][n], A, tb.dV[1][q][n] * B);
+      kp[n]     = pos_part(k);
       kmax      = fmax(kmax, fabs(k));
       sumkp     = sumkp + kp[n];
     }
-    // beta_n = K+_n / sum K+ (FP64 inverse in both precisions); w_q detJ beta_n is e K+_n
-    const double e = wj * (1.0 / double(sumkp));
-
-    const double erq = e * rq;
-#pragma unroll
-    for (int n = 0; n < NDOF; ++n)
-      lda[n] += erq * double(kp[n]);
+    // FP64 inverse in both precisions
+    const double e = wj * rcp_fast(double(sumkp));
+    double tkd     = 0.0;
     if (SCHEME != RDS_PGLDA)
     {
-      // sum_{m != n} K+_m (u_n - u_m) = u_n sum_m K+_m - sum_m K+_m u_m (the m = n terms
-      // cancel), so the N dissipation costs O(ndof) per point instead of O(ndof^2)
-      double tku = 0.0;
 #pragma unroll
-      for (int m = 0; m < NDOF; ++m)
-        tku += double(kp[m]) * ud[m];
-      const double sk = double(sumkp);
-#pragma unroll
-      for (int n = 0; n < NDOF; ++n)
-        diss[n] += (e * double(kp[n])) * (ud[n] * sk - tku);
+      for (int m = 1; m < NDOF; ++m)
+        tkd += double(kp[m]) * d[m];
     }
+    const double e1 = SPLIT ? e * rq : e * (rq - tkd);
+    const double ex = e * tkd;
+#pragma unroll
+    for (int n = 0; n < NDOF; ++n)
+    {
+      acc1[n] += e1 * double(kp[n]);
+      if (SCHEME == RDS_PGB)
+        accx[n] += ex * double(kp[n]);
+      if (SCHEME != RDS_PGLDA)
+        accw[n] += wj * double(kp[n]);
+    }
+  }
+  // PGN, PGPSI: lda is the whole residual, diss zero
+  double lda[NDOF], diss[NDOF];
+#pragma unroll
+  for (int n = 0; n < NDOF; ++n)
+  {
+    lda[n]  = SPLIT ? acc1[n] : fma(d[n], accw[n], acc1[n]);
+    diss[n] = SCHEME == RDS_PGB ? fma(d[n], accw[n], -accx[n]) : 0.0;
   }
   // wave speed |K| max_{q,n} max(1e-6, |k_n|)
   const double wsc = vol * double(fmax(T(1.e-6), kmax));
+
+  int pos[NDOF];
+#pragma unroll
+  for (int n = 0; n < NDOF; ++n)
+    pos[n] = __ldg(a.out.pos + (size_t)n * a.ncells + c);
 
   double theta = 1.0;
   if (SCHEME == RDS_PGB)
@@ -236,8 +290,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
 
   // the record of local node n: residual and wave speed, at its place in the node's list
   auto put = [&](int n, double r) {
-    const int p = __ldg(a.out.pos + (size_t)n * a.ncells + c);
-    reinterpret_cast<double2 *>(a.out.rec)[p] = make_double2(r, wsc);
+    reinterpret_cast<double2 *>(a.out.rec)[pos[n]] = make_double2(r, wsc);
   };
   if (EXT && SCHEME == RDS_PGB && a.blend)
   {
@@ -247,13 +300,13 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
     {
-      tn[n] = __ldg(a.blend + __ldg(a.sol_conn + (size_t)n * a.ncells + c));
+      tn[n] = __ldg(a.blend + nodes.v[n]);
       tmax  = fmax(tmax, tn[n]);
     }
     const bool skip = tmax < 1.e-6;
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
-      put(n, skip ? lda[n] : lda[n] + tn[n] * diss[n]);
+      put(n, skip ? lda[n] : fma(tn[n], diss[n], lda[n]));
   }
   else if (SCHEME == RDS_PGPSI && fabs(phi) > 1.e-14)
   {
@@ -264,7 +317,7 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
     {
-      const double r = (lda[n] + diss[n]) / phi;
+      const double r = lda[n] / phi;
       x[n]           = (r < 0.0 ? 0.0 : r) + 1.e-12;
       sx += x[n];
     }
@@ -276,34 +329,41 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
   {
 #pragma unroll
     for (int n = 0; n < NDOF; ++n)
-      put(n, (SCHEME == RDS_PGLDA) ? lda[n] : lda[n] + theta * diss[n]);
+      put(n, SCHEME == RDS_PGB ? fma(theta, diss[n], lda[n]) : lda[n]);
   }
 }
 
-// FP64 P3 Burgers cells: capped at 128 registers (4 blocks per SM instead of 3; 11 % faster,
-// measured); 0 (no minimum) keeps the compiler's choice elsewhere (the cap slowed P3 advection)
-template <int PHYS, typename T, int NDOF>
-constexpr int kMinBlocks = (PHYS == RDS_BURGERS2D && NDOF >= 10 && sizeof(T) == 8) ? 4 : 0;
+// Blocks per SM asked of the register allocation (0: the compiler's choice). FP64 P3 Burgers: 4
+// (128 registers; 11 % faster than 3, while the cap slowed P3 advection). FP64 P2 PGB: 5 (96
+// registers, 32 bytes spilled; 47.2 us with the compiler's 108, 45.4 so on 524,288 cells).
+template <int PHYS, int SCHEME, typename T, int NDOF>
+constexpr int kMinBlocks = sizeof(T) != 8                              ? 0
+                           : PHYS == RDS_BURGERS2D && NDOF >= 10       ? 4
+                           : NDOF == 6 && SCHEME == RDS_PGB            ? 5
+                                                                       : 0;
 
 template <int PHYS, int SCHEME, typename T, int NDOF, int NQ, int NFL, int NGEO>
-__global__ void __launch_bounds__(kBlock, kMinBlocks<PHYS, T, NDOF>)
+__global__ void __launch_bounds__(kBlock, kMinBlocks<PHYS, SCHEME, T, NDOF>)
     cells_scalar2d(const __grid_constant__ CellArgs a,
                    const __grid_constant__ Tables<T, 2, NDOF, NQ, NFL, NGEO> tb)
 {
   pdl_wait_and_release();
-  if (*a.stop)
-    return;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c    = blockIdx.x * blockDim.x + threadIdx.x;
+  const int stop = *a.stop; // in flight with the index loads
   if (c >= a.ncells)
     return;
-  scalar_cell<PHYS, SCHEME, T, NDOF, NQ, NFL, NGEO>(a, tb, c);
+  CellNodes<NDOF, NGEO> nodes;
+  load_nodes(a, c, nodes);
+  if (stop)
+    return;
+  scalar_cell<PHYS, SCHEME, T, NDOF, NQ, NFL, NGEO>(a, tb, c, nodes);
 }
 
 // Batch form: a persistent grid walks the group's active tiles (the problems still iterating
 // at this precision); a tile is blockDim.x consecutive cells of one problem, so every thread of
 // a block maps to the same problem. Results per cell are those of cells_scalar2d.
 template <int PHYS, int SCHEME, typename T, int NDOF, int NQ, int NFL, int NGEO>
-__global__ void __launch_bounds__(128, kMinBlocks<PHYS, T, NDOF>)
+__global__ void __launch_bounds__(128, kMinBlocks<PHYS, SCHEME, T, NDOF>)
     cells_scalar2d_batch(const __grid_constant__ CellArgs a,
                          const __grid_constant__ Tables<T, 2, NDOF, NQ, NFL, NGEO> tb)
 {
@@ -326,7 +386,11 @@ __global__ void __launch_bounds__(128, kMinBlocks<PHYS, T, NDOF>)
     }
     const int c = a.bt.cbeg[lo] + (t - prefix[lo]) * (int)blockDim.x + (int)threadIdx.x;
     if (c < a.bt.cend[lo])
-      scalar_cell<PHYS, SCHEME, T, NDOF, NQ, NFL, NGEO, false>(a, tb, c);
+    {
+      CellNodes<NDOF, NGEO> nodes;
+      load_nodes(a, c, nodes);
+      scalar_cell<PHYS, SCHEME, T, NDOF, NQ, NFL, NGEO, false>(a, tb, c, nodes);
+    }
   }
 }
 

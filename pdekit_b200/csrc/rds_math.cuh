@@ -35,4 +35,18 @@ __device__ __forceinline__ double rsqrt_fast(double x)
 __device__ __forceinline__ float rcp_fast(float x) { return 1.f / x; }
 __device__ __forceinline__ float rsqrt_fast(float x) { return rsqrtf(x); }
 
+// max(0, x), and x < y of numbers that are not negative. FP64: integer tests, since a comparison
+// would take a slot of the FP64 pipe, which bounds these kernels.
+__device__ __forceinline__ double pos_part(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
+__device__ __forceinline__ float pos_part(float x) { return x > 0.f ? x : 0.f; }
+__device__ __forceinline__ bool less_pos(double x, double y)
+{
+  return __double_as_longlong(x) < __double_as_longlong(y);
+}
+__device__ __forceinline__ bool less_pos(float x, float y) { return x < y; }
+
+// x y, rounded (not fused into a sum that uses it).
+__device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
+__device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
+
 } // namespace rds
