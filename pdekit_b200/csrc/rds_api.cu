@@ -120,7 +120,15 @@ struct rds_ctx
   int n_if = 0, n_slots = 0;
 
   // pinned host scalars for the loop's stop test
-  int *h_stop = nullptr;
+  // what calls read back, in pinned memory: copies that do not synchronise one by one, and a norm
+  // that its kernel writes there
+  struct HostBack
+  {
+    int stop, iter;
+    unsigned status;
+    double norm[kMaxNeq], norm0[kMaxNeq];
+  };
+  HostBack *h_back = nullptr;
 
   // CUDA graphs: a chunk of fused iterations with FP64 cells (0), FP32 cells (1), batched
   // problems (2); one iteration without stop test for rds_run, FP64 (3) / FP32 (4) cells;
@@ -610,12 +618,8 @@ rds_status launch_residual_kernels(rds_ctx *ctx, const int *stop)
   return RDS_OK;
 }
 
-rds_status check_status(rds_ctx *ctx)
+rds_status status_of(rds_ctx *ctx, unsigned st)
 {
-  unsigned st = 0;
-  RDS_CUDA(cudaMemcpyAsync(&st, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-  RDS_CUDA(cudaStreamSynchronize(ctx->stream));
   if (st & kFlagNonFinite)
     return fail(ctx, RDS_ERR_NONFINITE, "non-finite residual norm");
   if (st & kFlagNegPressure)
@@ -623,6 +627,15 @@ rds_status check_status(rds_ctx *ctx)
   if (st & kFlagTimeout)
     return fail(ctx, RDS_ERR_CUDA, "a bounded device wait (tensor-core commit or fused-sweep barrier) gave up");
   return RDS_OK;
+}
+
+rds_status check_status(rds_ctx *ctx)
+{
+  unsigned st = 0;
+  RDS_CUDA(cudaMemcpyAsync(&st, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+  RDS_CUDA(cudaStreamSynchronize(ctx->stream));
+  return status_of(ctx, st);
 }
 
 void release_graph(rds_ctx *ctx)
@@ -1101,8 +1114,7 @@ rds_status rds_finalize(rds_ctx *ctx)
       (st = dalloc(ctx, &ctx->d_ws, N)) || (st = dalloc(ctx, &ctx->d_dt, N)) ||
       (st = dalloc(ctx, &ctx->d_vol, N)) || (st = dalloc(ctx, &ctx->d_inv_vol, N)) ||
       (NEQ == 1 && ((st = dalloc(ctx, &ctx->d_rec, (size_t)E * 2)) || (st = dalloc(ctx, &ctx->d_pos, S)))) ||
-      (NEQ > 1 && (st = dalloc(ctx, &ctx->d_val, (size_t)S * NEQ))) ||
-      (st = dalloc(ctx, &ctx->d_wsc, W)) ||
+      (NEQ > 1 && ((st = dalloc(ctx, &ctx->d_val, (size_t)S * NEQ)) || (st = dalloc(ctx, &ctx->d_wsc, W)))) ||
       (st = dalloc(ctx, &ctx->d_stage, (size_t)N * NEQ)) || (st = dalloc(ctx, &ctx->d_row, N + 1)) ||
       (st = dalloc(ctx, &ctx->d_ent_slot, E)) || (st = dalloc(ctx, &ctx->d_ent_ws, E)) ||
       (st = dalloc(ctx, &ctx->d_part, (size_t)(ctx->gblocks + 1) * NEQ)) || // +1: two node ranges
@@ -1111,7 +1123,7 @@ rds_status rds_finalize(rds_ctx *ctx)
       (st = dalloc(ctx, &ctx->d_zero, 1)) || (st = dalloc(ctx, &ctx->d_status, 1)) ||
       (st = dalloc(ctx, &ctx->d_counter, 1)))
     return st;
-  RDS_CUDA(cudaMallocHost(&ctx->h_stop, sizeof(int)));
+  RDS_CUDA(cudaMallocHost(&ctx->h_back, sizeof(rds_ctx::HostBack)));
   RDS_CUDA(cudaMemsetAsync(ctx->d_u, 0, (size_t)N * NEQ * sizeof(double), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_res, 0, (size_t)N * NEQ * sizeof(double), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_dt, 0, (size_t)N * sizeof(double), ctx->stream));
@@ -1120,9 +1132,10 @@ rds_status rds_finalize(rds_ctx *ctx)
   RDS_CUDA(cudaMemsetAsync(ctx->d_stop, 0, sizeof(int), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
   RDS_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
-  if (NEQ == 1)
-    RDS_CUDA(cudaMemsetAsync(ctx->d_rec, 0, (size_t)E * 2 * sizeof(double), ctx->stream));
-  RDS_CUDA(cudaMemsetAsync(ctx->d_wsc, 0, (size_t)W * sizeof(double), ctx->stream));
+  // cell volumes for the dual volumes: the wave speeds' place (one equation: the records', of
+  // which there are at least as many)
+  double *cvol = NEQ == 1 ? ctx->d_rec : ctx->d_wsc;
+  RDS_CUDA(cudaMemsetAsync(cvol, 0, (size_t)W * sizeof(double), ctx->stream));
   if ((st = upload(ctx, ctx->d_row, count.data(), N + 1)) ||
       (st = upload(ctx, ctx->d_ent_slot, ent_slot.data(), E)) ||
       (st = upload(ctx, ctx->d_ent_ws, ent_ws.data(), E)))
@@ -1130,8 +1143,7 @@ rds_status rds_finalize(rds_ctx *ctx)
   if (NEQ == 1) // where the cells and facets write their records
     RDS_CUDA(launch_entry_of_slot((int)E, ctx->d_ent_slot, ctx->d_pos, ctx->stream));
 
-  // Dual volumes: per-cell volume into the wave-speed slot space, then a gather (boundary
-  // slots hold zero).
+  // Dual volumes: per-cell volumes, then a gather (boundary slots hold zero).
   for (const HostCellGroup &g : ctx->groups)
   {
     // the cell's own-order rule when given (as the reference), else the residual rule
@@ -1146,20 +1158,17 @@ rds_status rds_finalize(rds_ctx *ctx)
         (st = upload(ctx, ddv, dvg.data(), dvg.size())))
       return st;
     RDS_CUDA(launch_cell_volume_raw(g.desc.ncells, d.dim, nqv, g.desc.ngeo, g.d_geo_conn,
-                                    ctx->d_X, d.ngeo_nodes, dw, ddv, ctx->d_wsc + g.ws_base,
+                                    ctx->d_X, d.ngeo_nodes, dw, ddv, cvol + g.ws_base,
                                     ctx->stream));
     RDS_CUDA(cudaStreamSynchronize(ctx->stream));
     cudaFree(dw);
     cudaFree(ddv);
   }
-  RDS_CUDA(launch_dual_volume(N, ctx->d_row, ctx->d_ent_ws, ctx->d_wsc, ctx->d_vol,
+  RDS_CUDA(launch_dual_volume(N, ctx->d_row, ctx->d_ent_ws, cvol, ctx->d_vol,
                               ctx->d_inv_vol, ctx->stream));
   RDS_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (NEQ == 1) // its wave speeds are in the records
-  {
-    cudaFree(ctx->d_wsc);
-    ctx->d_wsc = nullptr;
-  }
+  if (NEQ == 1)
+    RDS_CUDA(cudaMemsetAsync(ctx->d_rec, 0, (size_t)E * 2 * sizeof(double), ctx->stream));
   if ((st = dalloc(ctx, &ctx->d_loop, 1)) != RDS_OK ||
       (st = dalloc(ctx, &ctx->d_stall, 1)) != RDS_OK)
     return st;
@@ -1383,22 +1392,14 @@ rds_status rds_residual_norm(rds_ctx *ctx, double *norm)
   if (!ctx || !norm || !ctx->finalized)
     return ctx ? fail(ctx, RDS_ERR_INVALID, "not finalized or null") : RDS_ERR_INVALID;
   const int N = ctx->desc.nnodes, NEQ = ctx->desc.neq;
-  rds_status st = launch(ctx, [&](const char **name) {
-    *name = "norm_partials";
-    return launch_norm_partials(N, NEQ, ctx->d_res, ctx->d_dt, ctx->d_part, ctx->gblocks,
-                                ctx->stream);
+  const rds_status st = launch(ctx, [&](const char **name) {
+    return launch_norm(N, NEQ, ctx->d_res, ctx->d_dt, ctx->d_part, ctx->d_counter,
+                       ctx->h_back->norm, ctx->stream, name);
   });
   if (st != RDS_OK)
     return st;
-  st = launch(ctx, [&](const char **name) {
-    return launch_norm_final(ctx->d_part, ctx->gblocks, NEQ, N, ctx->d_norm, nullptr, nullptr,
-                             nullptr, 0, 0.0, nullptr, nullptr, ctx->stream, name);
-  });
-  if (st != RDS_OK)
-    return st;
-  RDS_CUDA(cudaMemcpyAsync(norm, ctx->d_norm, NEQ * sizeof(double), cudaMemcpyDeviceToHost,
-                           ctx->stream));
   RDS_CUDA(cudaStreamSynchronize(ctx->stream));
+  std::copy(ctx->h_back->norm, ctx->h_back->norm + NEQ, norm);
   return RDS_OK;
 }
 
@@ -2351,10 +2352,10 @@ static rds_status replay_chunks(rds_ctx *ctx, int gi, int nchunks, long long lau
     ctx->launches += launches_per_chunk;
     if (k + 1 < nchunks && (k % 4) == 3)
     {
-      RDS_CUDA(cudaMemcpyAsync(ctx->h_stop, ctx->d_stop, sizeof(int), cudaMemcpyDeviceToHost,
+      RDS_CUDA(cudaMemcpyAsync(&ctx->h_back->stop, ctx->d_stop, sizeof(int), cudaMemcpyDeviceToHost,
                                ctx->stream));
       RDS_CUDA(cudaStreamSynchronize(ctx->stream));
-      if (*ctx->h_stop)
+      if (ctx->h_back->stop)
         break;
     }
   }
@@ -2590,9 +2591,20 @@ rds_status rds_iterate(rds_ctx *ctx, double cfl, int max_iter, double drop, int 
       return st;
   }
   ctx->active_precision = ctx->desc.precision;
-  int done = 0;
-  RDS_CUDA(cudaMemcpyAsync(&done, ctx->d_iter, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  rds_ctx::HostBack &back = *ctx->h_back;
+  RDS_CUDA(cudaMemcpyAsync(&back.iter, ctx->d_iter, sizeof(int), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+  RDS_CUDA(cudaMemcpyAsync(&back.status, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+  if (drop > 0.0)
+  {
+    RDS_CUDA(cudaMemcpyAsync(back.norm, ctx->d_norm, NEQ * sizeof(double), cudaMemcpyDeviceToHost,
+                             ctx->stream));
+    RDS_CUDA(cudaMemcpyAsync(back.norm0, ctx->d_norm0, NEQ * sizeof(double),
+                             cudaMemcpyDeviceToHost, ctx->stream));
+  }
   RDS_CUDA(cudaStreamSynchronize(ctx->stream));
+  const int done = back.iter;
   if (it_done)
     *it_done = done;
   if (hist && done > 0)
@@ -2600,17 +2612,14 @@ rds_status rds_iterate(rds_ctx *ctx, double cfl, int max_iter, double drop, int 
     RDS_CUDA(cudaMemcpy(hist, ctx->d_hist, (size_t)done * NEQ * sizeof(double),
                         cudaMemcpyDeviceToHost));
   }
-  st = check_status(ctx);
+  st = status_of(ctx, back.status);
   if (st != RDS_OK)
     return st;
   if (drop > 0.0)
   {
-    std::vector<double> h((size_t)NEQ * 2);
-    RDS_CUDA(cudaMemcpy(h.data(), ctx->d_norm, NEQ * sizeof(double), cudaMemcpyDeviceToHost));
-    RDS_CUDA(cudaMemcpy(h.data() + NEQ, ctx->d_norm0, NEQ * sizeof(double), cudaMemcpyDeviceToHost));
     double rel = 0.0;
     for (int e = 0; e < NEQ; ++e)
-      rel = std::max(rel, h[NEQ + e] > 0 ? h[e] / h[NEQ + e] : 0.0);
+      rel = std::max(rel, back.norm0[e] > 0 ? back.norm[e] / back.norm0[e] : 0.0);
     if (rel > drop)
       return fail(ctx, RDS_ERR_ITER_CAP, "residual drop not reached within max_iter");
   }
@@ -3477,8 +3486,8 @@ rds_status rds_destroy(rds_ctx *ctx)
   for (void *p : bufs)
     if (p)
       cudaFree(p);
-  if (ctx->h_stop)
-    cudaFreeHost(ctx->h_stop);
+  if (ctx->h_back)
+    cudaFreeHost(ctx->h_back);
   for (TimingRec &r : ctx->trecs)
   {
     cudaEventDestroy(r.a);

@@ -348,28 +348,6 @@ __global__ void __launch_bounds__(kGBlock, gather_blocks_per_sm(NEQ))
   }
 }
 
-// Sum of (res * dt)^2 per block (compute_residual_norm outside the fused loop).
-template <int NEQ>
-__global__ void __launch_bounds__(kGBlock)
-    norm_partials(int nnodes, const double *res, const double *dt, double *part)
-{
-  __shared__ double smem[kGBlock / 32];
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll
-  for (int e = 0; e < NEQ; ++e)
-  {
-    double sq = 0.0;
-    if (v < nnodes)
-    {
-      const double r = __dmul_rn(res[(size_t)e * nnodes + v], dt[v]);
-      sq             = __dmul_rn(r, r);
-    }
-    const double s = block_sum<kGBlock>(sq, smem);
-    if (threadIdx.x == 0)
-      part[(size_t)blockIdx.x * NEQ + e] = s;
-  }
-}
-
 // Final reduction of the block partials in a fixed order, norm = sqrt(sum / N), the
 // iteration counter, the history and the device-side residual-drop / finiteness test.
 // Executed by one whole block (norm_final, or the last block of a fused gather).
@@ -442,6 +420,49 @@ __device__ void reduce_final(const double *part, int nblocks, int nnodes, double
         hist[(size_t)(it + j) * neq + e] = nv[e];
     *iter = it + m;
   }
+}
+
+// compute_residual_norm outside the fused loop: the norm of res dt with the chunk sums and the
+// last-block reduction of the fused gather.
+template <int NEQ>
+__global__ void __launch_bounds__(kGBlock)
+    norm_nodes(int nnodes, const double *__restrict__ res, const double *__restrict__ dt,
+               double *part, unsigned *counter, double *norm)
+{
+  __shared__ double smem[2][NEQ * (kGBlock / 32)];
+  __shared__ double nv[kMaxNeq];
+  __shared__ bool last;
+  const int nchunk = (nnodes + kGBlock - 1) / kGBlock;
+  int buf          = 0;
+  for (int chunk = blockIdx.x; chunk < nchunk; chunk += gridDim.x, buf ^= 1)
+  {
+    const int v = chunk * kGBlock + threadIdx.x;
+    double sq[NEQ];
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e)
+    {
+      const double r = v < nnodes ? __dmul_rn(res[(size_t)e * nnodes + v], dt[v]) : 0.0;
+      sq[e]          = __dmul_rn(r, r);
+    }
+    warp_sums<NEQ>(sq, smem[buf]);
+    __syncthreads();
+    if (threadIdx.x < NEQ)
+      part[(size_t)chunk * NEQ + threadIdx.x] = chunk_sum(smem[buf], threadIdx.x);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+  {
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last)
+    return;
+  __threadfence();
+  reduce_final<NEQ>(part, nchunk, nnodes, norm, nullptr, nullptr, nullptr, 0, 0.0, nullptr,
+                    nullptr, smem[0], nv);
+  if (threadIdx.x == 0)
+    *counter = 0u;
 }
 
 template <int NEQ>
@@ -872,19 +893,24 @@ cudaError_t launch_gather(const GatherArgs &a, int mode, int nblocks, cudaStream
   }
 }
 
-cudaError_t launch_norm_partials(int nnodes, int neq, const double *res, const double *dt,
-                                 double *part, int nblocks, cudaStream_t s)
+cudaError_t launch_norm(int nnodes, int neq, const double *res, const double *dt, double *part,
+                        unsigned *counter, double *norm, cudaStream_t s, const char **name)
 {
+  *name               = "residual_norm";
+  int grid            = 0;
+  const cudaError_t e = gather_grid(neq, (nnodes + kGBlock - 1) / kGBlock, &grid);
+  if (e != cudaSuccess)
+    return e;
   switch (neq)
   {
   case 1:
-    norm_partials<1><<<nblocks, kGBlock, 0, s>>>(nnodes, res, dt, part);
+    norm_nodes<1><<<grid, kGBlock, 0, s>>>(nnodes, res, dt, part, counter, norm);
     break;
   case 4:
-    norm_partials<4><<<nblocks, kGBlock, 0, s>>>(nnodes, res, dt, part);
+    norm_nodes<4><<<grid, kGBlock, 0, s>>>(nnodes, res, dt, part, counter, norm);
     break;
   case 5:
-    norm_partials<5><<<nblocks, kGBlock, 0, s>>>(nnodes, res, dt, part);
+    norm_nodes<5><<<grid, kGBlock, 0, s>>>(nnodes, res, dt, part, counter, norm);
     break;
   default:
     return cudaErrorInvalidValue;

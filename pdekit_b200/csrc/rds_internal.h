@@ -325,8 +325,10 @@ cudaError_t launch_norm_final(const double *part, int nblocks, int neq, int nnod
                               double *norm, double *norm0, double *hist, int *iter,
                               int max_hist, double drop, int *stop, unsigned *status,
                               cudaStream_t s, const char **name);
-cudaError_t launch_norm_partials(int nnodes, int neq, const double *res, const double *dt,
-                                 double *part, int nblocks, cudaStream_t s);
+// Residual norm in one launch: chunk sums into part, the last block their sum; norm may be pinned
+// host memory. counter is 0 before and after.
+cudaError_t launch_norm(int nnodes, int neq, const double *res, const double *dt, double *part,
+                        unsigned *counter, double *norm, cudaStream_t s, const char **name);
 cudaError_t launch_cell_volume_raw(int ncells, int dim, int nq, int ngeo, const int32_t *geo_conn,
                                    const double *X, int ngeo_nodes, const double *w,
                                    const double *dVgeo, double *cvol, cudaStream_t s);
