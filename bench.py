@@ -146,56 +146,61 @@ def barrier(world):
 
 def scalar_flops(physics, scheme, ndof, nq, nfl):
     """Scalar 2D kernel on straight-sided triangles (affine geometry), in the form the kernel
-    evaluates (flux contracted with invJ once per flux node, k_n = dV0 A + dV1 B):
+    evaluates (flux contracted with invJ once per flux node, k_n = dV0 A + dV1 B, the N part in
+    deviations d_n from the first dof as d_n W_n - X_n):
       flux nodes  nfl x (2 ndof - 1 + 2 + 6)        state at the node, flux, G0/G1 = invJ^T F
       geometry    28                                Jacobian, determinant, inverse
       per point   4 nfl - 1 + 4                     flux divergence, weight, volume, Phi
                   + (2 ndof - 1 for Burgers)        advection speed u_q
-                  + 6 + 6 ndof + 3                  A, B; k_n, K+, max |k|, sum K+; 1/sum, e
-                  + 2 ndof                          LDA part
-                  + (7 ndof for N / B)              N dissipation (O(ndof) form)
-      end         27 for B (blending), 5 otherwise
-    Configuration 2 (Burgers P2 B, ndof 6, nq 7, nfl 10): 1,316 flop; configuration 1
-    (advection P1 LDA, ndof 3, nq 6, nfl 6): 471 flop."""
+                  + 6 + 5 ndof + 3                  A, B; k_n, max |k|, sum K+; 1/sum, e
+                  + 2 ndof                          LDA part (N: with X)
+                  + (2 ndof for N, 4 ndof for B)    W_n (B: and X_n)
+                  + (2 (ndof - 1) + 1 for N / B)    sum K+ d
+      end         6 + 5 ndof + 9 for B (blending), ndof + 2 ndof + 5 for N, 5 for LDA
+    Configuration 2 (Burgers P2 B, ndof 6, nq 7, nfl 10): 1,243 flop; configuration 1
+    (advection P1 LDA, ndof 3, nq 6, nfl 6): 453 flop."""
     fl = nfl * (2 * ndof - 1 + 2 + 6) + 28
-    per_q = 4 * nfl - 1 + 4 + 6 + 6 * ndof + 3 + 2 * ndof
+    per_q = 4 * nfl - 1 + 4 + 6 + 5 * ndof + 3 + 2 * ndof
     if physics == "burgers":
         per_q += 2 * ndof - 1
     if scheme != "lda":
-        per_q += 7 * ndof
-    return fl + nq * per_q + (27 if scheme == "b" else 5)
+        per_q += (4 if scheme == "b" else 2) * ndof + 2 * (ndof - 1) + 1
+    end = {"lda": 5, "b": 15 + 5 * ndof}.get(scheme, 5 + 3 * ndof)
+    return fl + nq * per_q + end
 
 
 def euler_flops(dim, neq, ndof, nq, nfl, ngeo, scheme, const_jac=None):
     """Count of one Euler cell in the algorithm the kernel evaluates, each quantity counted once
-    (the kernel's second evaluation of the upwind factors and point states in its node pass is
-    not counted):
+    (the kernel's second evaluation of the upwind matrices in its node pass is not counted); D the
+    dimension:
       geometry    (1 if const_jac else nq) (2 D^2 ngeo + c_invJ)      c_invJ 10 (2D) / 60 (3D)
-      flux nodes  nfl (2 NEQ ndof + c_props + c_flux                  state, properties, flux
-                       + 2 NEQ D^2 if const_jac)                      flux contracted with invJ
+      flux nodes  nfl (2 NEQ ndof + 3 D + 9                           state; V, p, H
+                       + 2 D^2 if const_jac)                          contravariant mass flux
       points      nq (2 NEQ ndof                                      u_q
-                      + 2 NEQ D nfl (const_jac) or 2 NEQ D (D nfl + D)  flux divergence
-                      + c_props + c_ac + c_solve + 2)                 state, acoustic factors,
-                                                                      (sum K+)^-1 [r, sum K+ u]
-      point-node  nq ndof (2 D^2 + c_F + 4 NEQ^2 + NEQ + 11 NEQ       grad phi, upwind factors,
-                           + 24 NEQ for N / B)                        sum K+, K+ v (factored),
-                                                                      sum K+ du, K+ (u - u_bar)
-      c_props 20 / 22, c_flux 12 / 24, c_ac 15 / 17, c_F 58 / 69, c_solve 190 (adjugate) / 165
-      (LU) for 2D / 3D. const_jac defaults to straight-sided simplices.
-    Configuration 3: 54,786 (P3 triangle, 16 points) and 144,325 (P3 quadrilateral on the bump,
-    25 points); configuration 4: 52,116 (P2 tetrahedron, 14 points, LDA)."""
+                      + nfl (6 D + 2, or 2 D^2 + 6 D + 3) + 2 D^2     flux divergence
+                      + 5 D + 20 + c_solve (1 or 2) + 6 D + 10)       state, solves, to and from
+                                                                      the symmetrising variables
+      point-node  nq ndof (2 D^2 + 4 D + 18                           grad phi, normal, eigenvalues
+                           + 3 D + 2 + D (D + 1)                      sum K+
+                           + 8 D + 15                                 K+ v (PGN: v is in the next)
+                           + 11 D + 14 + 12 D + 24 for N / B)         sum K+ du, K+ (u - u_bar)
+      c_solve 20 + 14 (2D), 45 + 30 (3D) per right-hand side. const_jac defaults to straight-sided
+      simplices. Configuration 3: 34,027 (P3 triangle, 16 points) and 90,100 (P3 quadrilateral on
+      the bump, 25 points); configuration 4: 27,436 (P2 tetrahedron, 14 points, LDA)."""
     if const_jac is None:
         const_jac = (dim == 2 and ngeo == 3) or (dim == 3 and ngeo == 4)
-    c_invj, c_props, c_flux, c_ac, c_f, c_solve = (10, 20, 12, 15, 58, 190) if dim == 2 else \
-        (60, 22, 24, 17, 69, 165)
-    f = (1 if const_jac else nq) * (2 * dim * dim * ngeo + c_invj)
-    f += nfl * (2 * neq * ndof + c_props + c_flux + (2 * neq * dim * dim if const_jac else 0))
-    per_q = 2 * neq * ndof
-    per_q += 2 * neq * dim * nfl if const_jac else 2 * neq * dim * (dim * nfl + dim)
-    per_q += c_props + c_ac + c_solve + 2
-    per_qn = 2 * dim * dim + c_f + 4 * neq * neq + neq + 11 * neq
+    d = dim
+    c_invj, c_fac, c_rhs = (10, 20, 14) if d == 2 else (60, 45, 30)
+    f = (1 if const_jac else nq) * (2 * d * d * ngeo + c_invj)
+    f += nfl * (2 * neq * ndof + 3 * d + 9 + (2 * d * d if const_jac else 0))
+    per_q = 2 * neq * ndof + nfl * (6 * d + 2 if const_jac else 2 * d * d + 6 * d + 3)
+    per_q += 2 * d * d + 5 * d + 20 + 6 * d + 10
+    per_q += c_fac + c_rhs * (1 if scheme == "lda" else 2)
+    per_qn = 2 * d * d + 4 * d + 18 + 3 * d + 2 + d * (d + 1)
+    if scheme != "n":
+        per_qn += 8 * d + 15
     if scheme != "lda":
-        per_qn += 24 * neq
+        per_qn += 23 * d + 38
     return f + nq * per_q + nq * ndof * per_qn
 
 
