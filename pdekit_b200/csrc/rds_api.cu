@@ -181,6 +181,8 @@ struct rds_ctx
   int loop_pdl       = 0;
   double *d_ur = nullptr, *d_dres = nullptr, *d_dc_theta = nullptr;
   float *d_c32 = nullptr, *d_dtv = nullptr;
+  double *d_fbase    = nullptr; // facets' contributions of the exact sweep (BCArgs::base)
+  long long bc_slot0 = 0;       // first slot of the conditions
   // the correction sweeps of a cycle in one launch (dc_sweeps_fused) for meshes of at most
   // dc_fuse_cells cells (option "mixed_fuse_cells"; 0: separate launches); d_fbar its barrier
   long long dc_fuse_cells = 1LL << 16;
@@ -400,6 +402,7 @@ BCArgs bc_args(rds_ctx *ctx, const HostBC &b, const int *stop)
   a.gq         = b.d_gq;
   a.vol        = ctx->d_vol;
   a.out        = contrib(ctx, b.slot_base, b.ws_base);
+  a.base       = ctx->d_fbase ? ctx->d_fbase + (b.slot_base - ctx->bc_slot0) : nullptr;
   a.adv0       = ctx->desc.adv[0];
   a.adv1       = ctx->desc.adv[1];
   a.gamma      = ctx->desc.gamma;
@@ -1029,6 +1032,7 @@ rds_status rds_finalize(rds_ctx *ctx)
     S += (long long)g.desc.ndof * g.desc.ncells;
     W += g.desc.ncells;
   }
+  ctx->bc_slot0 = S;
   for (HostBC &b : ctx->bcs)
   {
     if (b.desc.kind == RDS_BC_STRONG_DIRICHLET)
@@ -1246,6 +1250,7 @@ rds_status rds_finalize(rds_ctx *ctx)
           (st = dalloc(ctx, &ctx->d_dres, N)) != RDS_OK ||
           (st = dalloc(ctx, &ctx->d_dtv, N)) != RDS_OK ||
           (st = dalloc(ctx, &ctx->d_c32, (size_t)S)) != RDS_OK ||
+          (st = dalloc(ctx, &ctx->d_fbase, (size_t)std::max(1LL, S - ctx->bc_slot0))) != RDS_OK ||
           (st = dalloc(ctx, &ctx->d_dc_theta, (size_t)nc)) != RDS_OK ||
           (st = dalloc(ctx, &ctx->d_fbar, 2)) != RDS_OK)
         return st;
@@ -1254,6 +1259,7 @@ rds_status rds_finalize(rds_ctx *ctx)
       ctx->extra.push_back(ctx->d_dres);
       ctx->extra.push_back(ctx->d_dtv);
       ctx->extra.push_back(ctx->d_c32);
+      ctx->extra.push_back(ctx->d_fbase);
       ctx->extra.push_back(ctx->d_dc_theta);
       RDS_CUDA(cudaMemsetAsync(ctx->d_dc_theta, 0, (size_t)nc * sizeof(double), ctx->stream));
       ctx->dc_ok = true;

@@ -280,13 +280,12 @@ __device__ __forceinline__ void bc_weak_facet(const BCArgs &a,
   if (NEQ == 1 && a.c32)
   {
     // correction sweep of the defect-correction loop: the change since the exact sweep, whose
-    // contribution is still in the record (FP64 difference, then FP32: relative to the change)
+    // contribution is in base (FP64 difference, then FP32: relative to the change)
 #pragma unroll
     for (int n = 0; n < NFDOF; ++n)
     {
-      const size_t i = (size_t)n * a.nfacets + f;
-      a.c32[a.out.slot_base + i] =
-          float(bres[n][0] - a.out.rec[(size_t)__ldg(a.out.pos + i) * 2]);
+      const long long i            = (long long)n * a.nfacets + f;
+      a.c32[a.out.slot_base + i] = float(bres[n][0] - a.base[i]);
     }
   }
   else
@@ -297,6 +296,8 @@ __device__ __forceinline__ void bc_weak_facet(const BCArgs &a,
       static_assert(NEQ == 1, "several equations: bc_points");
       const int p = __ldg(a.out.pos + (size_t)n * a.nfacets + f);
       reinterpret_cast<double2 *>(a.out.rec)[p] = make_double2(bres[n][0], a.vol[dof[n]] * coeff);
+      if (a.base)
+        a.base[(size_t)n * a.nfacets + f] = bres[n][0];
     }
   }
   if (bad)

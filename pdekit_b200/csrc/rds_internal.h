@@ -252,9 +252,11 @@ struct BCArgs
   const int *stop;
   double *u_strong; // strong Dirichlet: the state it overwrites (the same buffer as u)
   // correction sweep of the defect-correction loop (one equation): when set, the facet writes
-  // the change of its contribution since the exact sweep (still in its record) to c32[slot]
-  // instead of the record
+  // the change of its contribution since the exact sweep to c32[slot] instead of the record. base
+  // (contexts with that loop): the exact sweep's contributions, SoA [nfdof][nfacets], beside the
+  // records, whose two loads in a row would lengthen every fused correction sweep
   float *c32;
+  double *base;
 };
 
 struct GatherArgs
