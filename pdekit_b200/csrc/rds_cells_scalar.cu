@@ -155,8 +155,11 @@ __device__ __forceinline__ void scalar_cell(const CellArgs &a,
         F0 = T(a.adv0) * s;
         F1 = T(a.adv1) * s;
       }
-      G0[f] = fma(ij00, F0, ij10 * F1);
-      G1[f] = fma(ij01, F0, ij11 * F1);
+      // the product with F0 is the rounded one: Burgers' F0 = s^2 / 2 is the smaller of the two for
+      // |s| < 2 (residuals of P1 Burgers cells, LDA, off by 6.1e-16 of the largest in the mean
+      // square; 6.7e-16 with the other product rounded)
+      G0[f] = fma(ij10, F1, ij00 * F0);
+      G1[f] = fma(ij11, F1, ij01 * F0);
     }
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
