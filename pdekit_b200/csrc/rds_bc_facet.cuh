@@ -280,13 +280,17 @@ __device__ __forceinline__ void bc_weak_facet(const BCArgs &a,
   if (NEQ == 1 && a.c32)
   {
     // correction sweep of the defect-correction loop: the change since the exact sweep, whose
-    // contribution is in base (FP64 difference, then FP32: relative to the change)
+    // contribution is in base (FP64 difference, then FP32: relative to the change). All of base is
+    // read before the first store: a store between two loads may alias the second for all the
+    // compiler knows, and the loads, at the end of a fused sweep's longest thread, would wait for
+    // one another (20,000 P1 cells, Burgers, N: 4.76 -> 4.63 us a sweep)
+    double base[NFDOF];
 #pragma unroll
     for (int n = 0; n < NFDOF; ++n)
-    {
-      const long long i            = (long long)n * a.nfacets + f;
-      a.c32[a.out.slot_base + i] = float(bres[n][0] - a.base[i]);
-    }
+      base[n] = a.base[(size_t)n * a.nfacets + f];
+#pragma unroll
+    for (int n = 0; n < NFDOF; ++n)
+      a.c32[a.out.slot_base + (size_t)n * a.nfacets + f] = float(bres[n][0] - base[n]);
   }
   else
   {

@@ -386,9 +386,22 @@ __device__ __forceinline__ bool sweep_barrier(const DcFusedArgs &a)
     return fused_barrier(a.bar, a.wait_limit, a.test_extra);
 }
 
+// Blocks per SM of the grid form, asked of the register allocation (0: the compiler's choice). Its
+// threads are what the GPU holds at once, so a block less per SM is a second or third cell and node
+// a thread in every sweep, and left to itself the compiler moves P3 kernels between 3 blocks (168
+// registers) and 2 (207-255) with changes anywhere in the body. B200, a sweep of 45,000 P3 cells:
+// advection, N, 16 points, 12.4 us with 3 blocks and 17.9 with 2, Burgers, N, 13.2 and 20.1; 7,200
+// cells 7.9 and 8.5, 8.6 and 8.7. Burgers with LDA and 16 points would spill 404 bytes at 168
+// registers (7,200 cells 8.0 us, 7.8 with the compiler's 254) and keeps 2 blocks.
+constexpr int fused_blocks(int phys, int scheme, int ndof, int nq)
+{
+  const bool wide = phys == RDS_BURGERS2D && scheme == RDS_PGLDA; // the most registers a cell
+  return ndof == 3 ? 4 : ndof == 6 ? (wide ? 3 : 4) : wide && nq == 16 ? 0 : 3;
+}
+
 template <int PHYS, int SCHEME, int NDOF, int NQ, int NFL, int NFDOF, int NFQ, int NT,
           bool CLUSTER>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, CLUSTER ? 0 : fused_blocks(PHYS, SCHEME, NDOF, NQ))
     dc_sweeps_fused(const __grid_constant__ DcFusedArgs a,
                     const __grid_constant__ Tables<float, 2, NDOF, NQ, NFL, 3> tb,
                     const __grid_constant__ FusedFacetTables<NFDOF, NFQ> ft)

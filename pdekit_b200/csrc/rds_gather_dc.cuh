@@ -36,8 +36,8 @@ __device__ __forceinline__ void dc_correction_node(const GatherArgs &a, const in
   {
     float c[B];
 #pragma unroll
-    for (int k = 0; k < B; ++k) // past the end: the first of the four again
-      c[k] = dc_load_change<COHERENT>(a.c32 + __ldg(a.ent_slot + (i + k < i1 ? i + k : i)));
+    for (int k = 0; k < B; ++k) // nothing past the end: in a fused sweep each load is one of L2
+      c[k] = i + k < i1 ? dc_load_change<COHERENT>(a.c32 + __ldg(a.ent_slot + i + k)) : 0.f;
 #pragma unroll
     for (int k = 0; k < B; ++k)
       if (i + k < i1)
