@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(kGBlock, gather_blocks_per_sm(NEQ))
       gather_node<NEQ, DT, UPDATE, NORM, RK, DC>(a, v, cfl, sq);
     if (NORM)
     {
-      if (*a.stop) // uniform over the grid: only the last block of a launch sets it
+      // the same for every thread of the launch: its last block sets the flag, after every block
+      // has passed the barrier below with its last chunk (and has one: gather_grid)
+      if (*a.stop)
         return;
       warp_sums<NEQ>(sq, smem[buf]);
       __syncthreads(); // the other buffer is free again: its sums were read before this barrier
@@ -306,8 +308,6 @@ __global__ void __launch_bounds__(kGBlock, gather_blocks_per_sm(NEQ))
     // the norm needs no separate launch; no block ever waits for another
     __shared__ bool last;
     __shared__ double nv[kMaxNeq];
-    if (*a.stop)
-      return;
     if (NEQ > 1)
       __syncthreads(); // threads 0 .. NEQ - 1 have written the block's parts
     if (threadIdx.x == 0)
