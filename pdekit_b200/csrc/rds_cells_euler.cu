@@ -41,6 +41,7 @@
 
 #include "rds_internal.h"
 #include "rds_math.cuh"
+#include "rds_per_device.h"
 #include "rds_physics.cuh"
 
 namespace rds
@@ -963,21 +964,17 @@ cudaError_t launch_euler_one(const CellArgs &a, cudaStream_t s)
   constexpr int D = (PHYS == RDS_EULER3D) ? 3 : 2;
   using B         = EulerBlock<T, D, SCHEME, AFFINE, NDOF, NQ, NFL, NGEO, G>;
   auto k          = cells_euler<PHYS, SCHEME, T, NDOF, NQ, NFL, NGEO, AFFINE, G, B::NT>;
-  // the shared-memory opt-in is set once per instantiation (not a stream operation, so it
-  // also stays out of captured graphs)
-  static int nsm = 0;
-  if (nsm == 0)
-  {
-    int dev = 0, n = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess)
-      e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, B::BYTES);
-    if (e != cudaSuccess)
-      return e;
-    nsm = n;
-  }
+  // the shared-memory opt-in, once per instantiation and device (not a stream operation, so it
+  // also stays out of captured graphs), and the device's SMs
+  static PerDevice sms;
+  int nsm             = 0;
+  const cudaError_t e = sms.get(&nsm, [&](int dev, int *n) {
+    const cudaError_t f =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, B::BYTES);
+    return f != cudaSuccess ? f : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev);
+  });
+  if (e != cudaSuccess)
+    return e;
   const int units = (a.ncells + 32 / G - 1) / (32 / G);
   k<<<units < nsm ? units : nsm, B::NT, B::BYTES, s>>>(a);
   return cudaGetLastError();

@@ -23,6 +23,7 @@
 
 #include "rds_internal.h"
 #include "rds_math.cuh"
+#include "rds_per_device.h"
 #include "rds_tables.cuh"
 
 namespace rds
@@ -440,19 +441,19 @@ cudaError_t launch_batch_one(const HostCellGroup &g, const CellArgs &a, int grid
   fill_tables(tb, g.w, g.V, g.dV, g.dVgeo, g.dVf, g.Vsf);
   auto k = cells_scalar2d_batch<PHYS, SCHEME, T, NDOF, NQ, NFL, 3>;
   // a persistent grid only balances if all its CTAs are resident at once: cap it at the
-  // occupancy of this kernel and tile (computed once per tile size)
-  static int per_sm[2] = {0, 0}, nsm = 0;
-  const int ti = tile > 64 ? 1 : 0;
-  if (per_sm[ti] == 0)
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[ti], k, tile, 0);
-    if (per_sm[ti] < 1)
-      per_sm[ti] = 1;
-  }
-  const int cap = per_sm[ti] * nsm;
+  // occupancy of this kernel and tile (computed once per tile size and device)
+  static PerDevice resident[2];
+  int cap             = 0;
+  const cudaError_t e = resident[tile > 64 ? 1 : 0].get(&cap, [&](int dev, int *n) {
+    int nsm = 0, per_sm = 0;
+    cudaError_t f = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (f == cudaSuccess)
+      f = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tile, 0);
+    *n = (per_sm < 1 ? 1 : per_sm) * nsm;
+    return f;
+  });
+  if (e != cudaSuccess)
+    return e;
   k<<<grid < cap ? grid : cap, tile, 0, s>>>(a, tb);
   return cudaGetLastError();
 }

@@ -27,6 +27,7 @@
 #include "rds_bc_facet.cuh"
 #include "rds_gather_dc.cuh"
 #include "rds_internal.h"
+#include "rds_per_device.h"
 #include "rds_tables.cuh"
 
 namespace rds
@@ -502,23 +503,25 @@ cudaError_t launch_fused_one(const HostCellGroup &g, const HostBC *const *bcs,
     cfg.blockDim             = dim3(NTC);
     cfg.attrs                = attr;
     cfg.numAttrs             = 1;
-    // whether the cluster fits, asked once per kernel and process, on the device current at
-    // the first call (one device a process, as the library is used; the first call usually
-    // comes during a stream capture: the queries then run in relaxed capture mode and on no
-    // stream)
-    static int fits = -1;
-    if (fits < 0)
-    {
+    // whether the cluster fits (1; 2: not), asked once per kernel and device (the first call
+    // usually comes during a stream capture: the queries then run in relaxed capture mode and on
+    // no stream)
+    static PerDevice clusters;
+    int fits            = 0;
+    const cudaError_t e = clusters.get(&fits, [&](int, int *n) {
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
       cudaThreadExchangeStreamCaptureMode(&mode);
       int nclusters = 0;
-      cudaError_t e = cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveClusters(&nclusters, kc, &cfg);
-      fits = (e == cudaSuccess && nclusters >= 1) ? 1 : 0;
+      cudaError_t f = cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (f == cudaSuccess)
+        f = cudaOccupancyMaxActiveClusters(&nclusters, kc, &cfg);
+      *n = (f == cudaSuccess && nclusters >= 1) ? 1 : 2;
       cudaGetLastError();
       cudaThreadExchangeStreamCaptureMode(&mode);
-    }
+      return cudaSuccess;
+    });
+    if (e != cudaSuccess)
+      return e;
     if (fits == 1)
     {
       *cluster   = true;

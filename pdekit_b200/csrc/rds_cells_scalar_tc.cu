@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "rds_internal.h"
+#include "rds_per_device.h"
 #include "rds_tables.cuh"
 
 namespace rds
@@ -536,16 +537,15 @@ cudaError_t launch_tc_one(const HostCellGroup &g, const CellArgs &a, int grid, i
   using TD = TcDims<NDOF, NQ, NFL>;
   Tables<float, 2, NDOF, NQ, NFL, 3> tb;
   fill_tables(tb, g.w, g.V, g.dV, g.dVgeo, g.dVf, g.Vsf);
-  auto k               = cells_scalar2d_tc<PHYS, SCHEME, NDOF, NQ, NFL, BATCH>;
-  static bool attr_set = false;
-  if (!attr_set)
-  {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TD::SMEM);
-    if (e != cudaSuccess)
-      return e;
-    attr_set = true;
-  }
+  auto k = cells_scalar2d_tc<PHYS, SCHEME, NDOF, NQ, NFL, BATCH>;
+  static PerDevice opt_in;
+  int set              = 0;
+  const cudaError_t e  = opt_in.get(&set, [&](int, int *n) {
+    *n = 1;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TD::SMEM);
+  });
+  if (e != cudaSuccess)
+    return e;
   k<<<grid, kTcCells, TD::SMEM, s>>>(a, tb, g.d_tc, ntiles);
   return cudaGetLastError();
 }

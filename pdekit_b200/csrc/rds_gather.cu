@@ -12,6 +12,7 @@
 
 #include "rds_gather_dc.cuh"
 #include "rds_internal.h"
+#include "rds_per_device.h"
 
 namespace rds
 {
@@ -801,17 +802,13 @@ __global__ void __launch_bounds__(1024) batch_rebuild(const __grid_constant__ Re
 // 29.7 us, 25.5 with a block each).
 cudaError_t gather_grid(int neq, int nblocks, int *grid)
 {
-  static int nsm = 0;
-  if (nsm == 0)
-  {
-    int dev = 0, n = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess)
-      e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess)
-      return e;
-    nsm = n;
-  }
+  static PerDevice sms;
+  int nsm             = 0;
+  const cudaError_t e = sms.get(&nsm, [](int dev, int *n) {
+    return cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev);
+  });
+  if (e != cudaSuccess)
+    return e;
   const int most = nsm * gather_blocks_per_sm(neq);
   *grid          = nblocks < 2 * most ? nblocks : most;
   return cudaSuccess;
