@@ -591,10 +591,8 @@ __global__ void __launch_bounds__(NT, 1) cells_euler(const __grid_constant__ Cel
         const T P = T(gm1) * (uq[D + 1] - T(0.5) * uq[0] * v2);
         bad |= !(P > T(0));
         const T a2  = T(a.gamma) * (P * ir);
-        const T iaT = rsqrt_fast(a2);
-        aT          = a2 * iaT;
+        aT          = sqrt_and_inverse(a2, ia);
         ad          = double(aT);
-        ia          = sizeof(T) == 8 ? double(iaT) : rcp_fast(ad);
       }
       const double ga = gm1 * ia;
 

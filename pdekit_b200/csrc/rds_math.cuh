@@ -33,7 +33,20 @@ __device__ __forceinline__ double rsqrt_fast(double x)
 }
 
 __device__ __forceinline__ float rcp_fast(float x) { return 1.f / x; }
-__device__ __forceinline__ float rsqrt_fast(float x) { return rsqrtf(x); }
+
+// sqrt(x) for x > 0, and the reciprocal of the result in FP64. FP32: the correctly rounded root
+// (x rsqrtf(x) is off by up to 2 units in the last place).
+__device__ __forceinline__ double sqrt_and_inverse(double x, double &inv)
+{
+  inv = rsqrt_fast(x);
+  return x * inv;
+}
+__device__ __forceinline__ float sqrt_and_inverse(float x, double &inv)
+{
+  const float s = sqrtf(x);
+  inv           = rcp_fast(double(s));
+  return s;
+}
 
 // max(0, x), and x < y of numbers that are not negative. FP64: integer tests, since a comparison
 // would take a slot of the FP64 pipe, which bounds these kernels.
