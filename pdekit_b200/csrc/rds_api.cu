@@ -110,7 +110,10 @@ struct rds_ctx
   cudaEvent_t ev_in_ready[2] = {nullptr, nullptr}, ev_in_free[2] = {nullptr, nullptr};
   cudaEvent_t ev_out_ready[2] = {nullptr, nullptr}, ev_out_free[2] = {nullptr, nullptr};
   double *d_hin[2] = {nullptr, nullptr}, *d_hout[2] = {nullptr, nullptr};
-  double *d_hnorm[2] = {nullptr, nullptr};
+  // norms of the last kHostNorms steps: a step's norm is written before the wait for the downloads
+  // of the step two before it, so theirs must be another place (the third step's wait covers it)
+  static constexpr int kHostNorms = 4;
+  double *d_hnorm                 = nullptr; // [kHostNorms][neq]
   long long hstep = 0;
 
   // partitioned single mesh: the nodes this rank shares with others, their slots in the
@@ -1952,11 +1955,10 @@ static rds_status step_host_init(rds_ctx *ctx)
     RDS_CUDA(cudaEventCreateWithFlags(&ctx->ev_out_free[k], cudaEventDisableTiming));
     rds_status st;
     if ((st = dalloc(ctx, &ctx->d_hin[k], n)) != RDS_OK ||
-        (st = dalloc(ctx, &ctx->d_hout[k], n)) != RDS_OK ||
-        (st = dalloc(ctx, &ctx->d_hnorm[k], (size_t)ctx->desc.neq)) != RDS_OK)
+        (st = dalloc(ctx, &ctx->d_hout[k], n)) != RDS_OK)
       return st;
   }
-  return RDS_OK;
+  return dalloc(ctx, &ctx->d_hnorm, (size_t)rds_ctx::kHostNorms * ctx->desc.neq);
 }
 
 rds_status rds_step_host(rds_ctx *ctx, const double *u_in, double *u_out, double cfl, double *norm)
@@ -1969,6 +1971,7 @@ rds_status rds_step_host(rds_ctx *ctx, const double *u_in, double *u_out, double
     return st;
   const int N = ctx->desc.nnodes, NEQ = ctx->desc.neq;
   const size_t bytes = (size_t)N * NEQ * sizeof(double);
+  double *dnorm      = ctx->d_hnorm + (size_t)(ctx->hstep % rds_ctx::kHostNorms) * NEQ;
   const int k        = (int)(ctx->hstep++ & 1);
   cudaStream_t s     = ctx->stream;
 
@@ -1989,7 +1992,7 @@ rds_status rds_step_host(rds_ctx *ctx, const double *u_in, double *u_out, double
   if ((st = rds_run(ctx, cfl, 1)) != RDS_OK)
     return st;
   st = launch(ctx, [&](const char **name) {
-    return launch_norm_final(ctx->d_part, ctx->gblocks, NEQ, N, ctx->d_hnorm[k], nullptr,
+    return launch_norm_final(ctx->d_part, ctx->gblocks, NEQ, N, dnorm, nullptr,
                              nullptr, nullptr, 0, 0.0, nullptr, nullptr, s, name);
   });
   if (st != RDS_OK)
@@ -2007,7 +2010,7 @@ rds_status rds_step_host(rds_ctx *ctx, const double *u_in, double *u_out, double
   RDS_CUDA(cudaStreamWaitEvent(ctx->h_out, ctx->ev_out_ready[k], 0));
   RDS_CUDA(cudaMemcpyAsync(u_out, ctx->d_hout[k], bytes, cudaMemcpyDeviceToHost, ctx->h_out));
   if (norm)
-    RDS_CUDA(cudaMemcpyAsync(norm, ctx->d_hnorm[k], NEQ * sizeof(double), cudaMemcpyDeviceToHost,
+    RDS_CUDA(cudaMemcpyAsync(norm, dnorm, NEQ * sizeof(double), cudaMemcpyDeviceToHost,
                              ctx->h_out));
   RDS_CUDA(cudaEventRecord(ctx->ev_out_free[k], ctx->h_out));
   return RDS_OK;
@@ -3470,7 +3473,6 @@ rds_status rds_destroy(rds_ctx *ctx)
   {
     cudaFree(ctx->d_hin[k]);
     cudaFree(ctx->d_hout[k]);
-    cudaFree(ctx->d_hnorm[k]);
     for (cudaEvent_t e : {ctx->ev_in_ready[k], ctx->ev_in_free[k], ctx->ev_out_ready[k],
                           ctx->ev_out_free[k]})
       if (e)
@@ -3486,7 +3488,7 @@ rds_status rds_destroy(rds_ctx *ctx)
                   ctx->d_row,   ctx->d_ent_slot, ctx->d_ent_ws, ctx->d_part,   ctx->d_norm,
                   ctx->d_norm0, ctx->d_hist,  ctx->d_iter,    ctx->d_stop,     ctx->d_zero,
                   ctx->d_status, ctx->d_counter, ctx->d_loop, ctx->d_rk_u1, ctx->d_rk_u2,
-                  ctx->d_rk_res};
+                  ctx->d_rk_res, ctx->d_hnorm};
   for (void *p : ctx->extra)
     cudaFree(p);
   for (void *p : bufs)
