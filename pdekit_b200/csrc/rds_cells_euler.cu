@@ -25,9 +25,10 @@
 // in which the flux Jacobian in direction g = |g| n is symmetric and the entropy component is
 // decoupled: M^-1 K+ M = oc I + s (e0 e0^T + n n^T) + d (e0 n^T + n e0^T) on (y_0, y_V), oc on
 // the entropy, with lambda_c = |g| V.n, lambda_+- = |g| (V.n +- a), p = max(0, lambda_+) / 2,
-// m = max(0, lambda_-) / 2, oc = max(0, lambda_c), s = p + m - oc, d = p - m (the product
-// R max(0, Lambda) L of Euler2DCons.hpp:316-536 / Euler3DCons.hpp:332-560, exactly). A node's
-// part of sum K+ costs 9 FP64 operations in 2D (14 in 3D) after its eigenvalues instead of the 36
+// m = max(0, lambda_-) / 2, oc = max(0, lambda_c), s = p + m - oc, d = p - m: the product
+// R max(0, Lambda) L of Euler2DCons.hpp:316-536 / Euler3DCons.hpp:332-560 for |n| = 1. (In 2D the
+// reference leaves n = g below |g| = 1e-9, where the two differ by oc (1 - |n|^2) on the velocity's
+// diagonal: at most |g|^2 |V|, 1e-18 of a node's usual K+.) A node's part of sum K+ costs 9 FP64 operations in 2D (14 in 3D) after its eigenvalues instead of the 36
 // (55) of two full rank-one terms with their factors, and the sum is solved as a symmetric
 // positive definite 3 x 3 (4 x 4) system and a scalar instead of a general 4 x 4 (5 x 5) one.
 // What bounds them: the FP64 pipe (B200, ncu: 61 % busy on the P2 tetrahedra, the issue slots 52 %,
@@ -937,11 +938,15 @@ __global__ void __launch_bounds__(NT, 1) cells_euler(const __grid_constant__ Cel
 }
 
 // One block per SM with all of its shared memory. Warps: 16 (128 registers a thread) where the
-// cells' regions and the tables fit and a lane has at most 12 accumulators; with more of them the
-// 128 registers spill inside the loops, and 12 warps of 168 are faster (P3 hybrid mesh, PGB, 16
-// accumulators and more: 165 us a launch against 176; P2 triangles, PGN, 8 accumulators: 27 us
-// with 12 warps, 23 with 16); fewer where 12 do not fit. NT stays a multiple of 64: 14 warps get
-// the registers of 16.
+// cells' regions and the tables fit and a lane has at most 12 accumulators, 12 of 168 otherwise,
+// fewer where 12 do not fit. Both sides measured, us a launch on B200, 12 warps against 16. More
+// accumulators: P3 hybrid mesh, PGB, 165 against 176. At most 12 (24,000 triangles, 16,000
+// quadrilaterals): P2 triangles, PGN, 47 against 45; P1, P2 and P3 quadrilaterals, PGN, 25, 44 and
+// 115 against 22, 39 and 111; level are P3 triangles, PGN, and P3 quadrilaterals, PGLDA, 25 points
+// (95), and with 20 points these take 78 against 80. That holds although some spill at 128
+// registers: 116 bytes stored by PGN on P2 quadrilaterals, 272 by PGLDA on P3 quadrilaterals, whose
+// lanes keep the sums of 4 points in phase C. NT stays a multiple of 64: 14 warps get the
+// registers of 16.
 template <typename T, int D, int SCHEME, bool AFFINE, int NDOF, int NQ, int NFL, int NGEO, int G>
 struct EulerBlock
 {

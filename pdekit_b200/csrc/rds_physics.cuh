@@ -42,22 +42,6 @@ __device__ __forceinline__ bool euler_props(const T *u, T gamma, EulerProps<T, D
   return !(p.P > T(0));
 }
 
-// Physical flux F[e][d] at one point.
-template <typename T, int D>
-__device__ __forceinline__ void euler_flux(const T *u, const EulerProps<T, D> &p, T F[][D])
-{
-#pragma unroll
-  for (int d = 0; d < D; ++d)
-  {
-    const T m = u[1 + d]; // rho * V_d
-    F[0][d]   = m;
-#pragma unroll
-    for (int k = 0; k < D; ++k)
-      F[1 + k][d] = m * p.V[k] + (k == d ? p.P : T(0));
-    F[D + 1][d] = m * p.H;
-  }
-}
-
 // Flux through direction n: F(u) . n (Euler2DCons::flux(p, direction, flux),
 // physics/euler/Euler2DCons.hpp:253-266; Euler3DCons.hpp:267-285).
 template <typename T, int D>

@@ -5,8 +5,9 @@
 // each table entry is consumed directly as a constant-bank operand of the FMA that needs it: no
 // load instruction, no shared-memory traffic, and the same entry is broadcast to all threads of
 // a warp (every thread works on a different cell of the same element type). The tables of the
-// largest element type used here (P3 quadrilateral, 20 quadrature points, P4 flux basis) take
-// 20 KB in FP64, inside the 32 KB parameter limit of CUDA 12.1+ on sm_70 and newer.
+// largest element type that travels so (the element Jacobians' P3 quadrilateral, 20 quadrature
+// points, P4 flux basis) take 20 KB in FP64, inside the 32 KB parameter limit of CUDA 12.1+ on sm_70
+// and newer; the Euler residual cells stage theirs in shared memory.
 #pragma once
 
 #include <cstring>
