@@ -250,11 +250,11 @@ def group_work(prob):
 # DRAM bytes (read + write) per launch of the dominant cell kernel(s) of a workload, from one ncu
 # capture of the same kernel (cold caches between replays); the summary files give the command.
 PROFILED_TRAFFIC = {
-    "c1": (0.30771e6, "profiles/dram_traffic_cell_kernels.md"),
+    "c1": (0.411136e6, "profiles/dram_traffic_cell_kernels.md"),
     "c2": (44.133888e6 + 5.847296e6, "profiles/cells_burgers_b_p2_512.md"),
-    "c3": ((102.96 + 119.78 + 192.94 + 217.37) * 1e6,  # both groups, per iteration
-           "profiles/cells_euler_c3_c4.md"),
-    "c4": ((91.06 + 268.62) * 1e6, "profiles/cells_euler_c3_c4.md"),
+    "c3": ((102.83 + 119.73 + 192.84 + 213.79) * 1e6,  # both groups, per iteration
+           "profiles/dram_traffic_cell_kernels.md"),
+    "c4": ((91.09 + 268.99) * 1e6, "profiles/dram_traffic_cell_kernels.md"),
 }
 
 
